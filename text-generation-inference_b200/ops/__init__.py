@@ -332,9 +332,17 @@ def has_fused_sample(scores) -> bool:
     return use_native(scores)
 
 
-def fused_sample(scores, temperature=None, top_k=None, top_p=None, do_sample=None, seeds=None, steps=None, typical_p=None):
-    """One-kernel temperature / top-k / top-p / typical-p / sampling on CUDA tensors (see ``ops.cuda.fused_sample``)."""
-    return native().fused_sample(scores, temperature, top_k, top_p, do_sample, seeds, steps, typical_p=typical_p)
+def fused_sample(scores, temperature=None, top_k=None, top_p=None, do_sample=None, seeds=None, steps=None, typical_p=None,
+                 history=None, repetition_penalty=None):
+    """One-kernel repetition penalty / temperature / top-k / top-p / typical-p / sampling on CUDA tensors (see
+    ``ops.cuda.fused_sample``)."""
+    return native().fused_sample(scores, temperature, top_k, top_p, do_sample, seeds, steps, typical_p=typical_p,
+                                 history=history, repetition_penalty=repetition_penalty)
+
+
+def fused_sample_penalises(scores) -> bool:
+    """Whether ``fused_sample`` takes the repetition penalty for these scores (otherwise ``penalties`` comes first)."""
+    return scores.dtype in (torch.float32, torch.bfloat16) and scores.shape[1] <= native().SAMPLE_PENALTY_MAX_VOCAB
 
 
 def penalties(scores, history, repetition_penalty=None, frequency_penalty=None):

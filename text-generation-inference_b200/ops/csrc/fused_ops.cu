@@ -18,7 +18,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "sampling.cuh"
 #include "launch.cuh"
 
 namespace {
@@ -509,231 +508,6 @@ argmax_logprob_kernel(const T* __restrict__ logits, long long* __restrict__ ids,
 
 
 // ------------------------------------------------------------------------------------------------
-// Fused sampler: temperature, top-k, top-p, Gumbel-max sampling (or argmax) and the log-probability of
-// the chosen token, one CTA per row.  Replaces the reference's chain of logits warpers and its
-// `probs / Exp(1)` multinomial with a CPU generator per request (utils/tokens.py:346-399,
-// utils/logits_process.py:25-358): no sort, no [B, V] probability matrix, no host round trip.
-//
-//   x_j = logit_j / T
-//   top-k: keep x_j >= (k-th largest x);  top-p: keep x_j unless the mass of strictly larger entries
-//   already reaches p (same sets as the sort-based torch filters).  Both thresholds are found by
-//   bisection on the order-preserving integer image of the float, which is exact and needs no sort.
-//   sample: argmax_j (x_j + g_j) over the kept set, g_j = -log(-log u_j), u_j from Philox4x32-10
-//   keyed by the request's seed with counter (j, step): reproducible for a given seed.
-//   logprob = x_c - logsumexp over the kept set.
-// ------------------------------------------------------------------------------------------------
-using tgi_sampling::gumbel_noise;
-using tgi_sampling::order_bits;
-
-// Calls f(index, score / T) for every entry of a row, the CTA's threads striding over it; 16-byte loads where the
-// row allows it (8 bf16 or 4 fp32 per thread and step).
-template <typename T, typename F>
-__device__ __forceinline__ void scan_row(const T* __restrict__ row, int V, float inv_t, F&& f) {
-  constexpr int VEC = 16 / sizeof(T);
-  const int nvec = (reinterpret_cast<uintptr_t>(row) & 15) == 0 ? V / VEC : 0;
-  for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-    const uint4 raw = reinterpret_cast<const uint4*>(row)[v];
-    const T* e = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) f(v * VEC + j, static_cast<float>(e[j]) * inv_t);
-  }
-  for (int i = nvec * VEC + threadIdx.x; i < V; i += blockDim.x) f(i, static_cast<float>(row[i]) * inv_t);
-}
-
-// smallest order_bits threshold t such that  sum_{x : bits(x) > t} w(x) < limit   (w = 1 or exp(x - m)),
-// not below floor_bits and not above the bits of the row maximum.
-// Radix select over the four bytes of the ordered bits, most significant first: one pass over the row per byte
-// builds a 256-bin histogram of the weights of the entries that match the bytes found so far, and a walk down
-// the bins finds the byte of t (the lowest bin whose entries can still be left out).  Five passes replace the
-// 32 of a bisection.  Weights are accumulated as 2^-40 fixed point in 64-bit integers, so the sums do not depend
-// on the order in which the lanes' atomics land: the same row always yields the same threshold.
-constexpr int kHistCopies = 16;          // one histogram per pair of warps (1024 threads)
-constexpr float kFixedOne = 1099511627776.f;   // 2^40
-
-template <typename T, bool MASS>
-__device__ uint32_t find_threshold(const T* __restrict__ row, int V, float inv_t, float m, float limit, uint32_t floor_bits,
-                                   unsigned long long* hist, unsigned long long* tot) {
-  const unsigned long long lim = MASS ? static_cast<unsigned long long>(fmaxf(limit, 0.f) * kFixedOne)
-                                      : static_cast<unsigned long long>(fmaxf(limit, 0.f));
-  const int copy = (threadIdx.x >> 5) % kHistCopies;
-  uint32_t prefix = 0u;
-  unsigned long long above = 0ull;         // weight of the entries whose leading bytes exceed the prefix
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    for (int i = threadIdx.x; i < kHistCopies * 256; i += blockDim.x) hist[i] = 0ull;
-    __syncthreads();
-    const uint32_t hi_mask = shift == 24 ? 0u : (0xffffffffu << (shift + 8));
-    unsigned int* hist32 = reinterpret_cast<unsigned int*>(hist);      // counts fit 32 bits: the cheaper atomic
-    scan_row(row, V, inv_t, [&](int, float x) {
-      const uint32_t b = order_bits(x);
-      if (b >= floor_bits && (b & hi_mask) == prefix) {
-        if (MASS) atomicAdd(&hist[copy * 256 + ((b >> shift) & 255u)], static_cast<unsigned long long>(__expf(x - m) * kFixedOne));
-        else atomicAdd(&hist32[copy * 256 + ((b >> shift) & 255u)], 1u);
-      }
-    });
-    __syncthreads();
-    if (threadIdx.x < 256) {
-      unsigned long long t = 0ull;
-#pragma unroll
-      for (int c = 0; c < kHistCopies; ++c)
-        t += MASS ? hist[c * 256 + threadIdx.x] : static_cast<unsigned long long>(reinterpret_cast<unsigned int*>(hist)[c * 256 + threadIdx.x]);
-      tot[threadIdx.x] = t;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      // S(v) = above + sum of the bins over v is the weight left out when t ends in bin v; S(255) < lim holds on
-      // entry, and going one bin down adds that bin: stop before the sum would reach lim
-      unsigned long long run = above;
-      int v = 255;
-      while (v > 0 && run + tot[v] < lim) {
-        run += tot[v];
-        --v;
-      }
-      tot[256] = run;
-      tot[257] = static_cast<unsigned long long>(v);
-    }
-    __syncthreads();
-    above = tot[256];
-    prefix |= static_cast<uint32_t>(tot[257]) << shift;
-    __syncthreads();
-  }
-  return max(min(prefix, order_bits(m)), floor_bits);
-}
-
-// Typical-p (utils/logits_process.py:389-448): over the entries the earlier filters kept, with p_j their
-// renormalised probabilities and H their entropy, keep the entries with the smallest |-log p_j - H| whose mass
-// reaches `mass`.  Returns the largest kept deviation as float bits (deviations are >= 0, so their bit patterns
-// order like the values); found by bisection, no sort.
-template <typename T>
-__device__ uint32_t typical_threshold(const T* __restrict__ row, int V, float inv_t, float m, uint32_t keep_from, float mass,
-                                      float* red, float* log_z_out, float* entropy_out) {
-  float z = 0.f;
-  scan_row(row, V, inv_t, [&](int, float x) {
-    if (order_bits(x) >= keep_from && x != -INFINITY) z += __expf(x - m);
-  });
-  const float log_z = __logf(block_sum(z, red));
-  float h = 0.f;
-  scan_row(row, V, inv_t, [&](int, float x) {
-    if (order_bits(x) >= keep_from && x != -INFINITY) {
-      const float lp = x - m - log_z;
-      h -= __expf(lp) * lp;
-    }
-  });
-  const float H = block_sum(h, red);
-  *log_z_out = log_z;
-  *entropy_out = H;
-  uint32_t lo = 0u, hi = 0x7f800000u;       // predicate "mass of deviations <= t reaches `mass`": true at +inf
-  while (lo < hi) {
-    const uint32_t mid = lo + ((hi - lo) >> 1);
-    float acc = 0.f;
-    scan_row(row, V, inv_t, [&](int, float x) {
-      if (order_bits(x) >= keep_from && x != -INFINITY) {
-        const float lp = x - m - log_z;
-        if (__float_as_uint(fabsf(-lp - H)) <= mid) acc += __expf(lp);
-      }
-    });
-    if (block_sum(acc, red) >= mass) hi = mid;
-    else lo = mid + 1;
-  }
-  return lo;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(1024)
-sample_kernel(const T* __restrict__ scores, long long row_stride, const float* __restrict__ temperature,
-              const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ typical_p,
-              const unsigned char* __restrict__ do_sample,
-              const long long* __restrict__ seeds, const int* __restrict__ steps, long long* __restrict__ ids,
-              float* __restrict__ logprob, int V) {
-  tgi::pdl_wait();      // inputs come from earlier kernels of the stream
-  tgi::pdl_trigger();   // let the next kernel be placed while this one runs
-  __shared__ float red[32];
-  __shared__ float s_val[32];
-  __shared__ int s_idx[32];
-  __shared__ unsigned long long s_hist[kHistCopies * 256];
-  __shared__ unsigned long long s_tot[258];
-  const int b = blockIdx.x;
-  const T* row = scores + static_cast<size_t>(b) * row_stride;
-  const float temp = temperature != nullptr ? temperature[b] : 1.f;
-  const float inv_t = 1.f / (temp > 0.f ? temp : 1.f);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // ---- max ----
-  float m = -INFINITY;
-  scan_row(row, V, inv_t, [&](int, float x) { m = fmaxf(m, x); });
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  __syncthreads();
-  if (lane == 0) red[warp] = m;
-  __syncthreads();
-  m = red[0];
-  for (int w = 1; w < (blockDim.x >> 5); ++w) m = fmaxf(m, red[w]);
-  __syncthreads();
-  // ---- thresholds ----
-  uint32_t keep_from = 0u;                      // keep entries whose order_bits >= keep_from
-  const int k = top_k != nullptr ? top_k[b] : 0;
-  if (k > 0 && k < V) keep_from = find_threshold<T, false>(row, V, inv_t, m, static_cast<float>(k), 0u, s_hist, s_tot);
-  const float p = top_p != nullptr ? top_p[b] : 1.f;
-  if (p < 1.f) {
-    float z = 0.f;
-    scan_row(row, V, inv_t, [&](int, float x) {
-      if (order_bits(x) >= keep_from) z += __expf(x - m);
-    });
-    z = block_sum(z, red);
-    const uint32_t t = find_threshold<T, true>(row, V, inv_t, m, p * z, keep_from, s_hist, s_tot);
-    keep_from = max(keep_from, t);
-  }
-  const float typ = typical_p != nullptr ? typical_p[b] : 1.f;
-  uint32_t typ_bits = 0xffffffffu;
-  float typ_log_z = 0.f, typ_h = 0.f;
-  if (typ < 1.f) typ_bits = typical_threshold<T>(row, V, inv_t, m, keep_from, typ, red, &typ_log_z, &typ_h);
-  // ---- sample over the kept set ----
-  const bool sample = do_sample != nullptr && do_sample[b] != 0;
-  const uint64_t seed = seeds != nullptr ? static_cast<uint64_t>(seeds[b]) : 0ull;
-  const uint32_t step = steps != nullptr ? static_cast<uint32_t>(steps[b]) : 0u;
-  float z = 0.f, best = -INFINITY, best_x = 0.f;
-  int best_i = 0x7fffffff;
-  scan_row(row, V, inv_t, [&](int i, float x) {
-    if (order_bits(x) < keep_from || x == -INFINITY) return;
-    if (typ < 1.f && __float_as_uint(fabsf(-(x - m - typ_log_z) - typ_h)) > typ_bits) return;
-    z += __expf(x - m);
-    const float key = sample ? x + gumbel_noise(static_cast<uint32_t>(i), step, seed) : x;
-    if (key > best || (key == best && i < best_i)) {
-      best = key;
-      best_i = i;
-      best_x = x;
-    }
-  });
-  z = block_sum(z, red);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float k2 = __shfl_xor_sync(0xffffffffu, best, o);
-    const int i2 = __shfl_xor_sync(0xffffffffu, best_i, o);
-    const float x2 = __shfl_xor_sync(0xffffffffu, best_x, o);
-    if (k2 > best || (k2 == best && i2 < best_i)) {
-      best = k2;
-      best_i = i2;
-      best_x = x2;
-    }
-  }
-  __syncthreads();
-  if (lane == 0) {
-    red[warp] = best;
-    s_idx[warp] = best_i;
-    s_val[warp] = best_x;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (blockDim.x >> 5); ++w)
-      if (red[w] > best || (red[w] == best && s_idx[w] < best_i)) {
-        best = red[w];
-        best_i = s_idx[w];
-        best_x = s_val[w];
-      }
-    ids[b] = best_i == 0x7fffffff ? 0 : best_i;
-    logprob[b] = best_x - m - __logf(z);
-  }
-}
-
-// ------------------------------------------------------------------------------------------------
 // Repetition and frequency penalties on fp32 scores, in place, one CTA per row, from the row's token history
 // (reference: utils/logits_process.py:151-218).  `scores` may be a vocabulary slice [vocab_start,
 // vocab_start + V): ids outside the slice are skipped.  Repetition: every token of the history gets
@@ -975,22 +749,6 @@ int tgi_argmax_logprob(const void* logits, long long* ids, float* logprob, int B
   else
     tgi::launch(argmax_logprob_kernel<__nv_bfloat16>, dim3(B), dim3(1024), 0, stream, static_cast<const __nv_bfloat16*>(logits), ids,
                                                                  logprob, V, row_stride);
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
-}
-
-// Fused temperature / top-k / top-p / sampling; any of temperature, top_k, top_p, do_sample, seeds, steps may be
-// null (stage off).  `is_fp32` selects the element type of `scores`.
-int tgi_sample(const void* scores, long long row_stride, int is_fp32, const float* temperature, const int* top_k,
-               const float* top_p, const float* typical_p, const unsigned char* do_sample, const long long* seeds,
-               const int* steps, long long* ids, float* logprob, int B, int V, cudaStream_t stream) {
-  if (B <= 0) return 0;
-  if (V <= 0) return -10;
-  if (is_fp32)
-    tgi::launch(sample_kernel<float>, dim3(B), dim3(1024), 0, stream, static_cast<const float*>(scores), row_stride, temperature, top_k, top_p,
-                                                 typical_p, do_sample, seeds, steps, ids, logprob, V);
-  else
-    tgi::launch(sample_kernel<__nv_bfloat16>, dim3(B), dim3(1024), 0, stream, static_cast<const __nv_bfloat16*>(scores), row_stride, temperature,
-                                                         top_k, top_p, typical_p, do_sample, seeds, steps, ids, logprob, V);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

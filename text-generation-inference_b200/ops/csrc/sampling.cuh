@@ -25,13 +25,17 @@ __device__ __forceinline__ uint4 philox4x32(uint32_t c0, uint32_t c1, uint32_t k
   return make_uint4(c[0], c[1], c[2], c[3]);
 }
 
+__device__ __forceinline__ float gumbel_of(uint32_t w) {
+  const float u = (static_cast<float>(w >> 8) + 0.5f) * (1.0f / 16777216.0f);   // (0, 1)
+  return -__logf(-__logf(u));
+}
+
 // j is the index of the entry in the WHOLE vocabulary, so a vocabulary shard draws the same noise for its
 // entries as a single GPU that holds all of them
 __device__ __forceinline__ float gumbel_noise(uint32_t j, uint32_t step, uint64_t seed) {
   const uint4 r = philox4x32(j >> 2, step, static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
   const uint32_t w = (j & 3) == 0 ? r.x : (j & 3) == 1 ? r.y : (j & 3) == 2 ? r.z : r.w;
-  const float u = (static_cast<float>(w >> 8) + 0.5f) * (1.0f / 16777216.0f);   // (0, 1)
-  return -__logf(-__logf(u));
+  return gumbel_of(w);
 }
 
 }  // namespace tgi_sampling

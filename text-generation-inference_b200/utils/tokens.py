@@ -290,7 +290,10 @@ class NextTokenChooser:
         one kernel launch for the whole batch (``ops.fused_sample``)."""
         from .. import ops
 
-        if (self.any_rep or self.any_freq) and not self.watermarks and self.grammar is None and hasattr(ops, "penalties"):
+        inside = self.any_rep and not self.any_freq and not self.watermarks and self.grammar is None and ops.fused_sample_penalises(scores)
+        if inside:
+            pass                  # a repetition penalty alone goes with the sampling kernel: no fp32 copy of the scores
+        elif (self.any_rep or self.any_freq) and not self.watermarks and self.grammar is None and hasattr(ops, "penalties"):
             # penalties from the token history in one kernel (fp32 copy of the scores)
             scores = ops.penalties(scores, input_ids, self.repetition_penalty if self.any_rep else None,
                                    self.frequency_penalty if self.any_freq else None)
@@ -316,7 +319,8 @@ class NextTokenChooser:
         next_ids, next_logprobs = ops.fused_sample(
             scores, self.temperature if self.any_temperature else None, self.top_k if self.any_top_k else None,
             self.top_p if self.any_top_p else None, do_sample, seeds, steps,
-            typical_p=self.typical_p if self.any_typical else None)
+            typical_p=self.typical_p if self.any_typical else None,
+            history=input_ids if inside else None, repetition_penalty=self.repetition_penalty if inside else None)
         return next_ids, next_logprobs, None, torch.ones_like(next_ids), None
 
     def advance_grammar(self, next_ids: List[int]):
