@@ -1,0 +1,96 @@
+"""GEMMs of a few tokens (``ops/csrc/gemm_skinny_sm100.cu``): edges of blocks, units, walks and token tiles in the three weight
+formats against 64-bit products.
+
+Tolerance: the result is rounded to bf16 once (7 stored bits: half a unit is at most 2^-8 of the value) after fp32 sums,
+whose error is below 2^-16 of the sum of the products' magnitudes for the depths used here (2^-24 per addition, fewer than
+2^8 additions in a chain)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def dev():
+    return torch.device("cuda", 0)
+
+
+def _check(got, x, w, bias=None):
+    from tgi_b200.ops import cuda as K
+
+    torch.cuda.synchronize()
+    assert K.check_status(dev()) == 0, "a kernel wait timed out"
+    want = x @ w.t()
+    if bias is not None:
+        want = want + bias.double()
+    bound = want.abs() * 2 ** -8 + (x.abs() @ w.abs().t() + 1) * 2 ** -16
+    assert ((got.double() - want).abs() <= bound).all()
+
+
+TOKENS = [1, 8, 9, 16, 17, 24, 25, 32]
+
+
+@pytest.mark.parametrize("M", TOKENS)
+@pytest.mark.parametrize("N,Kd,ctas", [(8, 64, None), (40, 576, None), (200, 4096, 1), (1000, 1024, 3), (4096, 512, None)])
+def test_bf16(M, N, Kd, ctas):
+    from tgi_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    wide = torch.randn(M, Kd + 64, device=dev(), generator=g).to(torch.bfloat16)
+    w = (torch.randn(N, Kd, device=dev(), generator=g) * 0.05).to(torch.bfloat16)
+    bias = torch.randn(N, device=dev(), generator=g).to(torch.bfloat16)
+    x = wide[:, :Kd].contiguous()
+    _check(K.gemm_bf16(x, w, bias, max_ctas=ctas), x.double(), w.double(), bias)
+    x = wide[:, 16:16 + Kd]                      # read in place from the wider matrix
+    _check(K.gemm_bf16(x, w, max_ctas=ctas), x.double(), w.double())
+
+
+@pytest.mark.parametrize("M", [1, 7, 8])
+@pytest.mark.parametrize("N,Kd,ctas", [(8, 128, None), (200, 1152, None), (1000, 2048, 3), (4096, 1024, None)])
+def test_fp8(M, N, Kd, ctas):
+    from tgi_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    xq, xs = K.fp8_quant_act(torch.randn(M, Kd, device=dev(), generator=g).to(torch.bfloat16))
+    wq = (torch.randn(N, Kd, device=dev(), generator=g) * 60).clamp(-440, 440).to(torch.float8_e4m3fn)
+    ws = torch.exp2(torch.randint(-12, -6, ((N + 127) // 128, Kd // 128), device=dev(), generator=g).float())
+    x = (xq.double().view(M, -1, 128) * xs.double()[:, :, None]).view(M, Kd)
+    w = (wq.double().view(N, -1, 128) * ws.double().repeat_interleave(128, 0)[:N, :, None]).view(N, Kd)
+    _check(K.gemm_fp8_block(xq, xs, wq, ws, max_ctas=ctas), x, w)
+
+
+@pytest.mark.parametrize("M", TOKENS)
+@pytest.mark.parametrize("N,Kd,group,zero", [(8, 256, 128, True), (200, 2304, 128, True), (1000, 2048, 256, True),
+                                             (4096, 512, 128, False), (264, 1024, 1024, True)])
+def test_int4(M, N, Kd, group, zero):
+    from tgi_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, Kd, device=dev(), generator=g).to(torch.bfloat16)
+    wq = torch.randint(0, 256, (N, Kd // 2), device=dev(), dtype=torch.uint8, generator=g)
+    scale = (torch.rand(Kd // group, N, device=dev(), generator=g) * 0.02 + 0.002).to(torch.float16)
+    zp = torch.randint(0, 17, (Kd // group, N), device=dev(), generator=g).to(torch.float16) if zero else None
+    bias = torch.randn(N, device=dev(), generator=g).to(torch.bfloat16)
+    q = torch.stack([wq & 15, wq >> 4], -1).view(N, Kd // group, group).double()
+    z = zp.t().double()[:, :, None] if zero else 8.0
+    w = ((q - z) * scale.t().double()[:, :, None]).view(N, Kd)
+    got = K.gemm_wq(x, wq, scale, zp, group, 4, bias)
+    # the sums are of (128 + q) x with 128 + z times the tokens' sum taken off: products up to 144 instead of 16 scales
+    torch.cuda.synchronize()
+    assert K.check_status(dev()) == 0, "a kernel wait timed out"
+    want = x.double() @ w.t() + bias.double()
+    mag = x.double().abs() @ (144 * scale.double().abs().repeat_interleave(group, 0))
+    assert ((got.double() - want).abs() <= want.abs() * 2 ** -8 + (mag + 1) * 2 ** -16).all()
+
+
+def test_full_ring_gives_the_same_result_every_time():
+    """32 tokens keep the consumers busier than the weights' copies: a stage given back before its last shared load has
+    returned shows as a result that changes from call to call."""
+    from tgi_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(0)
+    x = torch.randn(32, 14336, device=dev(), generator=g).to(torch.bfloat16)
+    w = (torch.randn(4096, 14336, device=dev(), generator=g) * 0.02).to(torch.bfloat16)
+    first = K.gemm_bf16(x, w)
+    _check(first, x.double(), w.double())
+    for _ in range(20):
+        assert torch.equal(K.gemm_bf16(x, w), first)

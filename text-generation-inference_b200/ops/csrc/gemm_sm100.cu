@@ -9,6 +9,8 @@
 // Replaces, in the reference, cuBLAS `F.linear` (layers/linear.py:44) and the fp8 paths
 // `w8a8_block_fp8_matmul` / `cutlass_scaled_mm` / `torch._scaled_mm` (layers/fp8.py:507-579).
 //
+// A few tokens (bf16 up to 16 or 32, fp8 up to 8) go to gemm_skinny_sm100.cu.
+//
 // Tile: 128 tokens x 256 weight rows per CTA for M <= 128.  For M > 128 two CTAs of a cluster work
 // as a pair (`cta_group::2`) on 256 tokens x 256 weight rows: each CTA loads its own 128 tokens and
 // one half of the 256 weight rows, the even CTA issues MMAs of 256 x 256 that read the weight
@@ -51,6 +53,7 @@
 // initialisation and before TMEM is freed, on every path, error paths included.
 #include <atomic>
 
+#include "gemm_skinny.h"
 #include "launch.cuh"
 #include "tensor_map.cuh"
 #include "sm100.cuh"
@@ -925,6 +928,8 @@ int tgi_gemm_bf16(const void* X, const void* W, void* C, const void* bias, int M
                   float* ws, int* counters, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K % 8 != 0) return -10;  // TMA row pitch must be a multiple of 16 bytes
+  if (tgi::skinny_bf16_applies(X, W, M, N, K, K, max_ctas))
+    return tgi::skinny_bf16(X, K, W, C, bias, M, N, K, max_ctas, status, stream);
   return dispatch<false>(X, nullptr, 0, W, nullptr, C, bias, M, N, K, K, max_ctas, ws, counters, status, stream, nullptr);
 }
 
@@ -933,6 +938,8 @@ int tgi_gemm_bf16_ld(const void* X, int ldx, const void* W, void* C, const void*
                      float* ws, int* counters, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K % 8 != 0 || ldx % 8 != 0 || ldx < K) return -10;
+  if (tgi::skinny_bf16_applies(X, W, M, N, K, ldx, max_ctas))
+    return tgi::skinny_bf16(X, ldx, W, C, bias, M, N, K, max_ctas, status, stream);
   return dispatch<false>(X, nullptr, 0, W, nullptr, C, bias, M, N, K, ldx, max_ctas, ws, counters, status, stream, nullptr);
 }
 
@@ -941,6 +948,8 @@ int tgi_gemm_fp8_block(const void* X, const float* xs_t, int xs_pitch, const voi
                        cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K % 128 != 0 || xs_pitch % 4 != 0) return -10;
+  if (tgi::skinny_fp8_applies(X, xs_t, W, M, K))
+    return tgi::skinny_fp8(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, max_ctas, status, stream);
   return dispatch<true>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, K, max_ctas, ws, counters, status, stream, nullptr);
 }
 

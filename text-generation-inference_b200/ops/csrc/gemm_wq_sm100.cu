@@ -11,7 +11,8 @@
 // weights stay packed in device memory (a 4-bit 70B model is 35 GB, not 140 GB) and a decode step streams a
 // quarter of the bytes of the bf16 GEMM.
 //
-// The tensor cores take bf16 operands from shared memory, so the weight tile is dequantised on its way there:
+// 4-bit weights of at most 32 tokens go to gemm_skinny_sm100.cu.  Otherwise:
+// the tensor cores take bf16 operands from shared memory, so the weight tile is dequantised on its way there:
 //   warp 0      TMA producer: token tile [128 x 64 bf16] with the 128-byte swizzle, and the RAW weight tile
 //               [128 rows x 32 or 64 bytes]
 //   warps 4-11  converters, half a weight row per thread: unpack, (q - zp) * scale in fp32, round to bf16 once (the
@@ -27,6 +28,7 @@
 
 #include <atomic>
 
+#include "gemm_skinny.h"
 #include "launch.cuh"
 #include "sm100.cuh"
 #include "tensor_map.cuh"
@@ -551,6 +553,8 @@ int tgi_gemm_wq(int bits, const void* X, void* Xh, const void* Wq, const void* s
                 cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K % kBK != 0 || group < kBK || group % kBK != 0 || N % 8 != 0 || ctas < 1) return -10;
+  if (bits == 4 && tgi::skinny_int4_applies(X, Wq, scale, zp, M, N, K, group))
+    return tgi::skinny_int4(X, Wq, scale, zp, group, C, bias, M, N, K, ctas, status, stream);
   if (bits == 4) return launch_wq<4>(X, Xh, Wq, scale, zp, group, C, partial, partial_floats, bias, M, N, K, ctas, status, stream);
   if (bits == 8) return launch_wq<8>(X, Xh, Wq, scale, nullptr, group, C, partial, partial_floats, bias, M, N, K, ctas, status, stream);
   return -11;
