@@ -94,3 +94,45 @@ def test_full_ring_gives_the_same_result_every_time():
     _check(first, x.double(), w.double())
     for _ in range(20):
         assert torch.equal(K.gemm_bf16(x, w), first)
+
+
+@pytest.mark.parametrize("fmt", ["bf16", "fp8", "int4"])
+def test_settled_weights_in_a_captured_step(fmt):
+    """Weights fetched while the kernel ahead still runs: a captured chain of norms and products gives, replay after replay, what the
+    same calls give in plain stream order."""
+    from tgi_b200.ops import cuda as K
+
+    H, M, L = 2048, 5, 6
+    g = torch.Generator(device="cuda").manual_seed(3)
+    norm = torch.ones(H, device=dev(), dtype=torch.bfloat16)
+    x = torch.randn(M, H, device=dev(), generator=g).to(torch.bfloat16)
+    ws = [torch.randn(H, H, device=dev(), generator=g) * 0.02 for _ in range(L)]
+    if fmt == "fp8":
+        ws = [((w * 2000).clamp(-440, 440).to(torch.float8_e4m3fn), torch.full((H // 128, H // 128), 2.0 ** -11, device=dev()))
+              for w in ws]
+    elif fmt == "int4":
+        ws = [(torch.randint(0, 256, (H, H // 2), device=dev(), dtype=torch.uint8, generator=g),
+               torch.full((H // 128, H), 0.004, device=dev(), dtype=torch.float16)) for _ in ws]
+    else:
+        ws = [w.to(torch.bfloat16) for w in ws]
+
+    def step(settled):
+        y = x
+        for w in ws:
+            if fmt == "fp8":
+                q, s, _ = K.rms_norm_quant(y, None, norm, 1e-5)
+                y = K.gemm_fp8_block(q, s, w[0], w[1], settled=settled)
+            else:
+                h, _ = K.rms_norm(y, None, norm, 1e-5)
+                y = K.gemm_wq(h, w[0], w[1], None, 128, 4, settled=settled) if fmt == "int4" else K.gemm_bf16(h, w, settled=settled)
+        return y
+
+    want = step(False)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = step(True)
+    for _ in range(20):
+        got.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert K.check_status(dev()) == 0 and torch.equal(got, want)

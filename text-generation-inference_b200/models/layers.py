@@ -36,7 +36,7 @@ class FastLinear:
         return self.weight.shape[0]
 
     def __call__(self, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-        return ops.linear(x, self.weight, self.bias, out=out)
+        return ops.linear(x, self.weight, self.bias, out=out, settled=True)
 
 
 class PackedQuantLinear:
@@ -90,7 +90,7 @@ class PackedQuantLinear:
             x2 = x2.index_select(1, self.perm)
         if x2.is_cuda and ops.use_native(x2) and x2.dtype == torch.bfloat16:
             if x2.shape[0] <= self.fused_max_tokens:
-                y = ops.native().gemm_wq(x2, self.wq, self.scale, self.zp, self.group, self.bits, self.bias)
+                y = ops.native().gemm_wq(x2, self.wq, self.scale, self.zp, self.group, self.bits, self.bias, settled=True)
             else:
                 w = ops.native().wq_dequant_scratch(self.wq, self.scale, self.zp, self.group, self.bits, self.in_features)
                 y = ops.linear(x2, w, self.bias)
@@ -161,8 +161,8 @@ class Fp8Linear:
         if x_scale is None:
             x, x_scale = ops.fp8_quant_act(x)
         if self.channel_scale is None:
-            return ops.gemm_fp8_block(x, x_scale, self.qweight, self.scale, self.dtype, self.bias, out=out)
-        y = ops.gemm_fp8_block(x, x_scale, self.qweight, self.scale, self.dtype, None)
+            return ops.gemm_fp8_block(x, x_scale, self.qweight, self.scale, self.dtype, self.bias, out=out, settled=True)
+        y = ops.gemm_fp8_block(x, x_scale, self.qweight, self.scale, self.dtype, None, settled=True)
         # one elementwise kernel: the product is formed in fp32 (type promotion) and stored in the output dtype,
         # in place or straight into the caller's buffer
         dst = y if out is None else (out.fallback if getattr(out, "is_peer_push", False) else out)

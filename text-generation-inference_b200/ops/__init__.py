@@ -286,13 +286,13 @@ def _into(out, y):
     return out
 
 
-def linear(x, weight, bias=None, out=None):
-    """``x @ weight^T + bias``; ``out`` (bf16, contiguous) receives the result when given.  A weight with up to 7 more
+def linear(x, weight, bias=None, out=None, settled=False):
+    """``x @ weight^T + bias``; ``out`` (bf16, contiguous) receives the result when given; ``settled``: ``cuda.gemm_bf16``.  A weight with up to 7 more
     columns than ``x`` was padded at load to the 16-byte rows the GEMM fetches."""
     if 0 < weight.shape[1] - x.shape[-1] < 8:
         x = torch.nn.functional.pad(x, (0, weight.shape[1] - x.shape[-1]))
     if use_native(x) and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16:
-        return native().gemm_bf16(x, weight, bias, out=out)
+        return native().gemm_bf16(x, weight, bias, out=out, settled=settled)
     return _into(out, ref.linear(x, weight, bias))
 
 
@@ -310,9 +310,9 @@ def fp8_quant_act(x, group=128):
     return ref.fp8_quant_act(x, group)
 
 
-def gemm_fp8_block(xq, xs, wq, ws, out_dtype=torch.bfloat16, bias=None, out=None):
+def gemm_fp8_block(xq, xs, wq, ws, out_dtype=torch.bfloat16, bias=None, out=None, settled=False):
     if use_native(xq):
-        return native().gemm_fp8_block(xq, xs, wq, ws, out_dtype, bias, out=out)
+        return native().gemm_fp8_block(xq, xs, wq, ws, out_dtype, bias, out=out, settled=settled)
     return _into(out, ref.gemm_fp8_block(xq, xs, wq, ws, out_dtype, bias))
 
 

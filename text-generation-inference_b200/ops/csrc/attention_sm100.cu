@@ -576,7 +576,7 @@ template <int D, bool FP8, bool KEEP>
 __global__ void __launch_bounds__(128)
 decode_kernel_v2(Params p) {
   tgi::pdl_wait();      // inputs come from earlier kernels of the stream
-  tgi::pdl_trigger();   // let the next kernel be placed while this one runs
+  tgi::pdl_release();   // let the next kernel be placed while this one runs
   extern __shared__ __align__(128) uint8_t smem[];
   using S = DecodeSmem<D, FP8>;
   constexpr int CT = S::CT;
@@ -801,7 +801,7 @@ template <class S>
 __global__ void __launch_bounds__(128, S::kMinBlocks)
 decode_kernel_v3(Params p, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
+  tgi::pdl_release();
   constexpr int D = S::D, CT = S::CT, MT = CT / 16, EB = S::EB;
   constexpr bool FP8 = S::FP8;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -1158,7 +1158,7 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_o, const floa
                                     const int* __restrict__ cu_seqlens_q, __nv_bfloat16* __restrict__ out, int Hq,
                                     int D, int nsplit, const float* sink) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
+  tgi::pdl_release();
   const int b = blockIdx.x, h = blockIdx.y;
   if (cu_seqlens_q[b + 1] == cu_seqlens_q[b]) return;
   const size_t base = (static_cast<size_t>(b) * Hq + h) * nsplit;

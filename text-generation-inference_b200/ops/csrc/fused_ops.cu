@@ -106,7 +106,7 @@ norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict
             __nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ res_out, uint8_t* __restrict__ q_out,
             float* __restrict__ scale_t, int scale_pitch, int H, float eps, float w_offset) {
   tgi::pdl_wait();      // inputs come from earlier kernels of the stream
-  tgi::pdl_trigger();   // let the next kernel be placed while this one runs
+  tgi::pdl_release();   // let the next kernel be placed while this one runs
   __shared__ float red[32];
   const int row = blockIdx.x;
   const size_t base = static_cast<size_t>(row) * H;
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(256)
 act_mul_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, uint8_t* __restrict__ q_out,
                float* __restrict__ scale_t, int scale_pitch, int I, int act) {
   tgi::pdl_wait();      // inputs come from earlier kernels of the stream
-  tgi::pdl_trigger();   // let the next kernel be placed while this one runs
+  tgi::pdl_release();   // let the next kernel be placed while this one runs
   constexpr int E = 8 * NV;            // elements per thread
   constexpr int LANES = 128 / E;       // lanes per quantisation group
   const int row = blockIdx.y;
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(256)
 quant_act_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q_out, float* __restrict__ scale_t,
                  int scale_pitch, int K) {
   tgi::pdl_wait();      // inputs come from earlier kernels of the stream
-  tgi::pdl_trigger();   // let the next kernel be placed while this one runs
+  tgi::pdl_release();   // let the next kernel be placed while this one runs
   const int row = blockIdx.y;
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = v < K / 8;

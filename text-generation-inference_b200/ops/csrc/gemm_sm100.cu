@@ -929,27 +929,28 @@ int tgi_gemm_bf16(const void* X, const void* W, void* C, const void* bias, int M
   if (M <= 0 || N <= 0) return 0;
   if (K % 8 != 0) return -10;  // TMA row pitch must be a multiple of 16 bytes
   if (tgi::skinny_bf16_applies(X, W, M, N, K, K, max_ctas))
-    return tgi::skinny_bf16(X, K, W, C, bias, M, N, K, max_ctas, status, stream);
+    return tgi::skinny_bf16(X, K, W, C, bias, M, N, K, max_ctas, 0, status, stream);
   return dispatch<false>(X, nullptr, 0, W, nullptr, C, bias, M, N, K, K, max_ctas, ws, counters, status, stream, nullptr);
 }
 
-// The same with rows of X `ldx` elements apart (X is a column slice of a wider matrix, 16-byte aligned).
-int tgi_gemm_bf16_ld(const void* X, int ldx, const void* W, void* C, const void* bias, int M, int N, int K, int max_ctas,
+// The same with rows of X `ldx` elements apart (X may be a column slice of a wider matrix, 16-byte aligned).  settled: W and bias
+// are not written by the launch that precedes this one on the stream (gemm_skinny.h); the same below.
+int tgi_gemm_bf16_ld(const void* X, int ldx, const void* W, void* C, const void* bias, int M, int N, int K, int max_ctas, int settled,
                      float* ws, int* counters, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K % 8 != 0 || ldx % 8 != 0 || ldx < K) return -10;
   if (tgi::skinny_bf16_applies(X, W, M, N, K, ldx, max_ctas))
-    return tgi::skinny_bf16(X, ldx, W, C, bias, M, N, K, max_ctas, status, stream);
+    return tgi::skinny_bf16(X, ldx, W, C, bias, M, N, K, max_ctas, settled, status, stream);
   return dispatch<false>(X, nullptr, 0, W, nullptr, C, bias, M, N, K, ldx, max_ctas, ws, counters, status, stream, nullptr);
 }
 
 int tgi_gemm_fp8_block(const void* X, const float* xs_t, int xs_pitch, const void* W, const float* wscale, void* C,
-                       const void* bias, int M, int N, int K, int max_ctas, float* ws, int* counters, int* status,
+                       const void* bias, int M, int N, int K, int max_ctas, int settled, float* ws, int* counters, int* status,
                        cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K % 128 != 0 || xs_pitch % 4 != 0) return -10;
   if (tgi::skinny_fp8_applies(X, xs_t, W, M, K))
-    return tgi::skinny_fp8(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, max_ctas, status, stream);
+    return tgi::skinny_fp8(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, max_ctas, settled, status, stream);
   return dispatch<true>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, K, max_ctas, ws, counters, status, stream, nullptr);
 }
 

@@ -546,15 +546,16 @@ int launch_wq(const void* X, void* Xh, const void* Wq, const void* scale, const 
 
 extern "C" {
 
+// settled: Wq, scale, zp and bias are not written by the launch that precedes this one on the stream (gemm_skinny.h)
 // bits: 4 (Wq uint8 [N, K / 2]) or 8 (Wq int8 [N, K]); scale / zp fp16 [K / group, N] (zp may be null: the 4-bit
 // zero point is then 8, the 8-bit format has none); partial: fp32 workspace of `partial_floats` floats or null.
 int tgi_gemm_wq(int bits, const void* X, void* Xh, const void* Wq, const void* scale, const void* zp, int group, void* C,
-                float* partial, long long partial_floats, const void* bias, int M, int N, int K, int ctas, int* status,
+                float* partial, long long partial_floats, const void* bias, int M, int N, int K, int ctas, int settled, int* status,
                 cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K % kBK != 0 || group < kBK || group % kBK != 0 || N % 8 != 0 || ctas < 1) return -10;
   if (bits == 4 && tgi::skinny_int4_applies(X, Wq, scale, zp, M, N, K, group))
-    return tgi::skinny_int4(X, Wq, scale, zp, group, C, bias, M, N, K, ctas, status, stream);
+    return tgi::skinny_int4(X, Wq, scale, zp, group, C, bias, M, N, K, ctas, settled, status, stream);
   if (bits == 4) return launch_wq<4>(X, Xh, Wq, scale, zp, group, C, partial, partial_floats, bias, M, N, K, ctas, status, stream);
   if (bits == 8) return launch_wq<8>(X, Xh, Wq, scale, nullptr, group, C, partial, partial_floats, bias, M, N, K, ctas, status, stream);
   return -11;

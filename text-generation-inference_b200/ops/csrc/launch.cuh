@@ -4,7 +4,8 @@
 // launched with the "programmatic stream serialization" attribute and starts with `pdl_wait()` (which
 // blocks until the kernels it depends on have completed and flushed their memory) followed by
 // `pdl_trigger()`, so the next kernel's CTAs can be placed on the SMs while this one is still
-// running.  Nothing is read or written before `pdl_wait()`, so stream-order semantics are preserved.
+// running.  Nothing is read or written before `pdl_wait()`, so stream-order semantics are preserved (but for settled weights,
+// see `pdl_release`).
 //
 // Measured on B200 (CUDA-graph decode step): Llama-3-70B fp8 at TP=1 56.6 ms with PDL against 56.4 ms
 // without, TP=2 35.4 against 34.8 ms, Llama-3-8B bf16 at TP=2 10.7 against 10.4 ms.  Inside a graph the
@@ -28,6 +29,12 @@ __device__ __forceinline__ void pdl_trigger() {
 #endif
 }
 
+// The trigger of the short kernels that a GEMM of a few tokens follows (norm, activation, quantisation, decode attention): such a
+// GEMM may be launched so that it fetches settled weights meanwhile (`launch_after`), and its CTAs take nothing that these
+// kernels' later CTAs need, since all of those have started when the trigger takes effect.  Comes after `pdl_wait()`, so that what
+// runs ahead of its own wait runs after everything but its direct predecessor.
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 inline bool pdl_enabled() {
   static const bool on = [] {
     const char* v = std::getenv("TGI_B200_PDL");
@@ -36,8 +43,10 @@ inline bool pdl_enabled() {
   return on;
 }
 
+// `early`: the kernel may be placed when all CTAs of its predecessor have triggered or ended; it calls `pdl_wait()` before it
+// touches anything that the predecessor reads or writes.
 template <typename... Params, typename... Args>
-inline cudaError_t launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+inline cudaError_t launch_after(bool early, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                           Args... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
@@ -48,8 +57,13 @@ inline cudaError_t launch(void (*kernel)(Params...), dim3 grid, dim3 block, size
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+template <typename... Params, typename... Args>
+inline cudaError_t launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return launch_after(pdl_enabled(), kernel, grid, block, smem, stream, args...);
 }
 
 // Same, with an optional thread-block cluster of `cluster_x` CTAs along x (1 = no cluster attribute).

@@ -220,8 +220,15 @@ def _gemm_ctas(lib, st, M: int, N: int, max_ctas: Optional[int]) -> int:
     return ctas
 
 
+def _settled(settled: bool, tokens: int) -> c_int:
+    """Whether the few-token GEMMs may fetch weights ahead of the stream's order.  Only inside a captured step: there the
+    launch ahead is a kernel of the step, and steps don't write weights."""
+    return c_int(1 if settled and tokens <= 32 and torch.cuda.is_current_stream_capturing() else 0)
+
+
 def gemm_bf16(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, max_ctas: Optional[int] = None,
-              out: Optional[torch.Tensor] = None):
+              out: Optional[torch.Tensor] = None, settled: bool = False):
+    """``settled``: the weights (and bias) belong to a layer and are never written by the launch right before the call."""
     lib = load()
     lead = x.shape[:-1]
     x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
@@ -252,9 +259,10 @@ def gemm_bf16(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = N
         return out.reshape(*lead, N)
     st = state(x.device)
     ctas = _gemm_ctas(lib, st, M, N, max_ctas)
-    if sliced:
-        _check(lib.tgi_gemm_bf16_ld(_ptr(x2), c_int(x2.stride(0)), _ptr(w), _ptr(out), _ptr(bias), c_int(M), c_int(N),
-                                    c_int(K), c_int(ctas), _ptr(st.ws), _ptr(st.counters), _ptr(st.status), _stream()),
+    early = _settled(settled, M)
+    if sliced or early.value:
+        _check(lib.tgi_gemm_bf16_ld(_ptr(x2), c_int(x2.stride(0) if sliced else K), _ptr(w), _ptr(out), _ptr(bias), c_int(M),
+                                    c_int(N), c_int(K), c_int(ctas), early, _ptr(st.ws), _ptr(st.counters), _ptr(st.status), _stream()),
                "gemm_bf16_ld")
         return out.reshape(*lead, N)
     _check(lib.tgi_gemm_bf16(_ptr(x2), _ptr(w), _ptr(out), _ptr(bias), c_int(M), c_int(N), c_int(K), c_int(ctas),
@@ -262,7 +270,8 @@ def gemm_bf16(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = N
     return out.reshape(*lead, N)
 
 
-def gemm_fp8_block(xq, xs, wq, ws, out_dtype=torch.bfloat16, bias=None, max_ctas: Optional[int] = None, out=None):
+def gemm_fp8_block(xq, xs, wq, ws, out_dtype=torch.bfloat16, bias=None, max_ctas: Optional[int] = None, out=None,
+                   settled: bool = False):
     lib = load()
     M, K = xq.shape
     N = wq.shape[0]
@@ -293,7 +302,7 @@ def gemm_fp8_block(xq, xs, wq, ws, out_dtype=torch.bfloat16, bias=None, max_ctas
     if not ws.is_contiguous():
         ws = ws.contiguous()
     _check(lib.tgi_gemm_fp8_block(_ptr(xq), c_void_p(sptr), c_int(pitch), _ptr(wq), _ptr(ws), _ptr(out), _ptr(bias),
-                                  c_int(M), c_int(N), c_int(K), c_int(ctas), _ptr(st.ws), _ptr(st.counters),
+                                  c_int(M), c_int(N), c_int(K), c_int(ctas), _settled(settled, M), _ptr(st.ws), _ptr(st.counters),
                                   _ptr(st.status), _stream()), "gemm_fp8_block")
     return out
 
@@ -892,7 +901,7 @@ def _wq_partial(device) -> torch.Tensor:
 
 
 def gemm_wq(x: torch.Tensor, wq: torch.Tensor, scale: torch.Tensor, zp: Optional[torch.Tensor], group: int, bits: int,
-            bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+            bias: Optional[torch.Tensor] = None, settled: bool = False) -> torch.Tensor:
     """``x[M, K] (bf16) @ dequant(wq)[N, K]^T`` with the weights dequantised on their way into shared memory:
     ``wq`` uint8 ``[N, K/2]`` (4-bit, low nibble first) or int8 ``[N, K]``; ``scale`` / ``zp`` fp16 ``[K/group, N]``."""
     lib = load()
@@ -905,7 +914,7 @@ def gemm_wq(x: torch.Tensor, wq: torch.Tensor, scale: torch.Tensor, zp: Optional
     xh = torch.empty(M, K, dtype=torch.float16, device=x.device)       # fp16 copy of the tokens, written by the call
     _check(lib.tgi_gemm_wq(c_int(bits), _ptr(x), _ptr(xh), _ptr(wq), _ptr(scale), _ptr(zp), c_int(group), _ptr(out),
                            _ptr(part), c_ll(part.numel()), _ptr(bias), c_int(M), c_int(N), c_int(K), c_int(st.sm_count),
-                           _ptr(st.status), _stream()), "gemm_wq")
+                           _settled(settled, M), _ptr(st.status), _stream()), "gemm_wq")
     return out
 
 
