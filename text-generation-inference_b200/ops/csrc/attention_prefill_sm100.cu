@@ -1,6 +1,6 @@
-// Paged causal prefill attention on the 5th-generation tensor cores (sm_100a): head size 128 (or, with bf16 pages, 192
-// for queries and keys), pages of 16 tokens, bf16 or e4m3 KV pages, ragged batches with a cached prefix (chunked
-// prefill), GQA, sliding window with kept first tokens, soft-capping, per-row horizons and a gate per token and head.
+// Paged causal prefill attention on the 5th-generation tensor cores (sm_100a), e4m3 pages of 16 tokens, and the entry points for all
+// pages (bf16: attention_prefill_bf16_sm100.cu).  Head size 128, ragged batches with a cached prefix (chunked prefill), GQA,
+// sliding window with kept first tokens, soft-capping and per-row horizons.
 //
 // Replaces, in the reference, flashinfer `BatchPrefillWithPagedKVCache` / FA2 `varlen_fwd`
 // (layers/attention/cuda.py:244-296, layers/attention/flashinfer.py:58-128).
@@ -18,9 +18,8 @@
 // K and V pages are fetched with TMA boxes of one page (16 tokens x 128 bytes) straight from the page pool, no
 // per-lane address arithmetic.  e4m3 pages are widened to fp16 (exact) on their way into the operand tiles by the
 // eight output warps, which are idle most of a tile (64 bytes per thread), and the MMAs then run in fp16 (Q is
-// converted once); bf16 pages feed bf16 MMAs directly.
-// Queries and keys of 192 take a third 64-element slab each; V and P are then single-buffered (V of the next tile is wanted
-// only after that tile's softmax, P is free again after the PV product, during the softmax's first pass).
+// converted once).  That widening sets the pace: the two chains of the bf16 kernel gave 4 to 10 % here (64 heads, 3300 tokens 475 ->
+// 456 us) and, with activations and KV quantised anew in every layer, changed a 70B model's prompts by as much as their error.
 // The S accumulator and the PV accumulator are double-buffered in TMEM (4 x 128 columns), so the tensor core
 // computes S of the next tile while the softmax warps work on the current one.
 // Every wait is bounded; a wait that runs out sets the status word, the CTA drains and frees its TMEM.
@@ -32,178 +31,40 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "attention_prefill.cuh"
 #include "launch.cuh"
-#include "sm100.cuh"
 #include "tensor_map.cuh"
 
-using namespace sm100;
+using namespace prefill;
 
 namespace {
 
-constexpr int kD = 128;            // value size of a head
-constexpr int kRows = 128;         // query rows per CTA
-constexpr int kKeys = 128;         // KV tokens per tile
-constexpr int kPage = 16;          // tokens per page
 constexpr int kThreads = 640;            // 20 warps: K producer, MMA, V producer, spare, 8 softmax, 8 output
-constexpr float kLog2e = 1.4426950408889634f;
-constexpr int kSlab = kRows * 128;             // bytes of one [128 rows x 128 bytes] swizzled slab
-constexpr int kTileBytes = 2 * kSlab;          // a 128 x 128 tile of 16-bit values: two slabs (32 KB)
+constexpr int kPolyEvery = 4;            // see `poly_exp2`
 
-struct PrefillParams {
-  const __nv_bfloat16* q;       // [T, Hq, 128 or 192]
-  const int* block_tables;      // [B, max_blocks]
-  const int* cu_seqlens_q;      // [B + 1]
-  const int* kv_lens;           // [B]
-  const float* k_scale;         // [Hkv] or null (e4m3 pages)
-  const float* v_scale;
-  __nv_bfloat16* out;           // [T, Hq, 128]
-  const int* horizon;           // optional [T]
-  const __nv_bfloat16* gate;    // optional [T, ld_gate]: the output of head h is multiplied by the sigmoid of column h
-  long long ld_gate;
-  int max_blocks, Hq, Hkv, num_blocks;
-  float scale, softcap;
-  int window;
-  int chunk;                    // > 0: a row sees only keys of its own chunk of `chunk` positions
-  int keep;                     // first tokens that every row sees whatever its window
-  const float* sink;            // [Hq] or null: score of one more key per head that has no value
-  int* status;
-};
-
-// First KV position that the query at `pos` may see.
-__device__ __forceinline__ int first_visible(const PrefillParams& p, int pos) {
-  int lo = p.window > 0 ? pos - p.window + 1 : 0;
-  if (p.chunk > 0 && pos > 0) lo = max(lo, pos - pos % p.chunk);
-  return max(lo, 0);
-}
-
-__device__ __forceinline__ void report(int* status, int code) {
-  if (status != nullptr) atomicCAS(status, 0, code);
-}
-
-// MN-major operand with the 128-byte swizzle (rows = K index, 128 bytes = 64 MN elements per row; groups of 8
-// rows 1024 bytes apart; the next 64 MN elements `lbo` bytes further): the layout TMA leaves a [tokens x head]
-// tile in.  Canonical form: cute/atom/mma_traits_sm100.hpp, make_umma_desc<Major::MN>.
-__device__ __forceinline__ uint64_t make_desc_mn_sw128(uint32_t smem_addr, uint32_t lbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFF) >> 4);
-  d |= static_cast<uint64_t>(lbo_bytes >> 4) << 16;
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
-}
-// instruction descriptor: D fp32, A K-major, B K-major or MN-major, fmt 0 = f16, 1 = bf16
-__device__ __forceinline__ constexpr uint32_t idesc16(uint32_t fmt, bool b_mn) {
-  return (1u << 4) | (fmt << 7) | (fmt << 10) | (0u << 15) | ((b_mn ? 1u : 0u) << 16) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
-}
-__device__ __forceinline__ uint32_t swz_chunk(int row, int chunk) { return static_cast<uint32_t>(row * 128 + ((chunk ^ (row & 7)) << 4)); }
-__device__ __forceinline__ float fast_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&r)[32]) {
-  tmem_ld_32x32b_x32(addr, r);
-  tmem_ld_wait(r);
-}
-
-// 2^x on the FMA pipe, for x <= 0: the special-function unit does 16 ex2 per cycle and SM and is the busiest
-// unit of a tile (16 K exponentials), so every kPolyEvery-th probability is computed this way instead.  Round x to
-// the nearest integer with the 1.5 * 2^23 trick, evaluate a cubic for 2^f on [-0.5, 0.5] (relative error 1.4e-4,
-// well under the 16-bit rounding of P) and add the integer to the exponent field.
-constexpr int kPolyEvery = 4;
-__device__ __forceinline__ float poly_exp2(float x) {
-  x = fmaxf(x, -125.f);
-  const float t = x + 12582912.f;
-  const float f = x - (t - 12582912.f);
-  float r = fmaf(0.05502927f, f, 0.24225698f);
-  r = fmaf(r, f, 0.69325305f);
-  r = fmaf(r, f, 0.99995134f);
-  return __int_as_float(__float_as_int(r) + (__float_as_int(t) << 23));
-}
-__device__ __forceinline__ float fast_tanh(float y) {      // 1 - 2 / (1 + e^(2y)); saturates cleanly at +-1
-  return 1.f - __fdividef(2.f, 1.f + fast_exp2(y * (2.f * kLog2e)));
-}
-// How a softmax thread reads its scores.  Key i of a 32-key group is visible when i - lo lies in [0, range]
-// (one unsigned compare); with soft-capping a raw score x becomes cap_out * tanh(x * cap_in), already in log2 units,
-// otherwise it is scaled by scale_log2 (> 0) — both after the maximum in the first pass, inside the FMA in the second.
-struct ScoreArgs {
-  float scale_log2, cap_in, cap_out;
-  int lo;
-  unsigned range;
-};
-template <bool MASK>
-__device__ __forceinline__ float group_max(const uint32_t (&v)[32], float mx, const ScoreArgs& a) {
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    float x = __uint_as_float(v[i]);
-    if (MASK) x = static_cast<unsigned>(i - a.lo) <= a.range ? x : -INFINITY;
-    mx = fmaxf(mx, x);
-  }
-  return mx;
-}
-// Probabilities of a 32-key group as sixteen packed 16-bit pairs (fp16 next to fp16 V tiles, bf16 otherwise);
-// returns their sum.  m is the row maximum in log2 units.
-template <bool MASK, bool CAP, bool F16>
-__device__ __forceinline__ float group_prob(const uint32_t (&v)[32], uint32_t (&packed)[16], float m, const ScoreArgs& a) {
-  float rs0 = 0.f, rs1 = 0.f;
-#pragma unroll
-  for (int i = 0; i < 32; i += 2) {
-    float pr[2];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const float x = __uint_as_float(v[i + e]);
-      if (CAP) pr[e] = fast_exp2(a.cap_out * fast_tanh(x * a.cap_in) - m);
-      else if (kPolyEvery > 0 && (i + e) % kPolyEvery == 1) pr[e] = poly_exp2(fmaf(x, a.scale_log2, -m));
-      else pr[e] = fast_exp2(fmaf(x, a.scale_log2, -m));
-      if (MASK) pr[e] = static_cast<unsigned>(i + e - a.lo) <= a.range ? pr[e] : 0.f;
-    }
-    rs0 += pr[0];
-    rs1 += pr[1];
-    if (F16) {
-      const __half2 hh = __floats2half2_rn(pr[0], pr[1]);
-      packed[i >> 1] = *reinterpret_cast<const uint32_t*>(&hh);
-    } else {
-      const __nv_bfloat162 bb = __floats2bfloat162_rn(pr[0], pr[1]);
-      packed[i >> 1] = *reinterpret_cast<const uint32_t*>(&bb);
-    }
-  }
-  return rs0 + rs1;
-}
-
-// Shared memory (bytes):  Q 32 K | K: bf16 2 x 32 K, e4m3 raw 2 x 16 K + converted 32 K | V: same | P 2 x 32 K | barriers;
-// with KS = 3 slabs of queries and keys:  Q 48 K | K 2 x 48 K | V 32 K | P 32 K | barriers
-template <bool FP8, int KS>
+// Shared memory (bytes):  Q 32 K | K raw 2 x 16 K + converted 32 K | V the same | P 2 x 32 K | barriers
 struct Layout {
-  static constexpr int kStagesVP = KS == 2 ? 2 : 1;               // of V and of P
   static constexpr int kQ = 0;
-  static constexpr int kK = KS * kSlab;
-  static constexpr int kKTile = KS * kSlab;
-  static constexpr int kV = kK + 2 * kKTile;                      // e4m3: 64 KB as well
-  static constexpr int kP = kV + kStagesVP * kTileBytes;
+  static constexpr int kK = kTileBytes;
+  static constexpr int kV = kK + 2 * kTileBytes;
+  static constexpr int kP = kV + 2 * kTileBytes;
   // two P tiles: the softmax of tile j + 1 writes one while the PV product of tile j still reads the other.  The
   // final partial row sums (float [2][128]) are written into the P tile that the last product does not read.
-  static constexpr int kBars = kP + kStagesVP * kTileBytes;
+  static constexpr int kBars = kP + 2 * kTileBytes;
   static constexpr int kAlpha = kBars + 256;                      // float [2][128]
   static constexpr int kRowMax = kAlpha + 2 * 128 * 4;            // float [2][128]: row maxima of the two halves
   static constexpr int kAbort = kRowMax + 2 * 128 * 4;            // int [4][2]: a softmax thread of the lane quarter gave up
-  static constexpr int kSums = kAbort + 64;                       // single-buffered P: the row sums' own place
   // no slack for aligning the base: the kernel checks that the dynamic shared memory starts on a 1024-byte
   // boundary (it does when the kernel has no static shared memory) and reports an error otherwise
-  static constexpr int kTotal = kSums + (kStagesVP == 1 ? 2 * 128 * 4 : 0);
+  static constexpr int kTotal = kAbort + 64;
   static_assert(kTotal <= 227 * 1024, "shared memory of a CTA");
-  // e4m3: raw stage s at kK + s * 16 K, converted tile at kK + 32 K
+  // raw stage s at kK + s * 16 K, converted tile at kK + 32 K
   static constexpr int kRawStage = kKeys * 128;
-  // stage and round of tile j
-  static __device__ __forceinline__ int stage(int j) { return kStagesVP == 2 ? j & 1 : 0; }
-  static __device__ __forceinline__ int round(int j) { return kStagesVP == 2 ? j >> 1 : j; }
 };
 
-template <bool FP8, int KS>
 __global__ void __launch_bounds__(kThreads, 1)
-prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const PrefillParams p) {
-  using L = Layout<FP8, KS>;
-  static_assert(KS == 2 || (KS == 3 && !FP8), "queries and keys of two slabs, or three of bf16");
+prefill_e4m3_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const PrefillParams p) {
+  using L = Layout;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if ((smem_u32(smem) & 1023u) != 0u) {       // uniform over the CTA, before anything is allocated
@@ -254,8 +115,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1);
       mbar_init(&v_full[i], 1);
-      mbar_init(&k_free[i], FP8 ? 8 : 1);      // e4m3: the eight converting warps
-      mbar_init(&v_free[i], FP8 ? 8 : 1);
+      mbar_init(&k_free[i], 8);      // the eight converting warps
+      mbar_init(&v_free[i], 8);
       mbar_init(&s_full[i], 1);
       mbar_init(&s_free[i], 8);
       mbar_init(&pv_full[i], 1);
@@ -296,7 +157,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   auto produce = [&](bool do_k, bool do_v) {
     bool ok = true;
     for (int j = 0; j < ntiles && ok; ++j) {
-      const int s = j & 1, vs = L::stage(j);
+      const int s = j & 1, vs = s;
       const int t0 = tile_start(j);
       int blk = 0;
       if (lane < kKeys / kPage) {
@@ -308,29 +169,21 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
       if (lane == 0) {
         if (do_k) {
           if (j >= 2) ok = mbar_wait(&k_free[s], ((j >> 1) - 1) & 1);
-          if (ok) mbar_arrive_expect_tx(&k_full[s], FP8 ? L::kRawStage : L::kKTile);
+          if (ok) mbar_arrive_expect_tx(&k_full[s], L::kRawStage);
         }
         if (do_v && ok) {
-          if (j >= L::kStagesVP) ok = mbar_wait(&v_free[vs], (L::round(j) - 1) & 1);
-          if (ok) mbar_arrive_expect_tx(&v_full[vs], FP8 ? L::kRawStage : kTileBytes);
+          if (j >= 2) ok = mbar_wait(&v_free[vs], ((j >> 1) - 1) & 1);
+          if (ok) mbar_arrive_expect_tx(&v_full[vs], L::kRawStage);
         }
         if (!ok) report(p.status, kErrProducerWait);
       }
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) break;
       const int pg = lane & 7;
-      if (FP8) {
-        // one 128-byte-wide box covers the whole head
-        if (lane < 8) {
-          if (do_k) tma_load_2d(smem + L::kK + s * L::kRawStage + pg * (kPage * 128), &tmK, &k_full[s], kvh * kD, blk * kPage);
-          if (do_v) tma_load_2d(smem + L::kV + s * L::kRawStage + pg * (kPage * 128), &tmV, &v_full[s], kvh * kD, blk * kPage);
-        }
-      } else {
-        const int hf = lane >> 3;                              // 64-element slab
-        if (do_k && hf < KS)
-          tma_load_2d(smem + L::kK + s * L::kKTile + hf * kSlab + pg * (kPage * 128), &tmK, &k_full[s], kvh * (64 * KS) + hf * 64, blk * kPage);
-        if (do_v && hf < 2)
-          tma_load_2d(smem + L::kV + vs * kTileBytes + hf * kSlab + pg * (kPage * 128), &tmV, &v_full[vs], kvh * kD + hf * 64, blk * kPage);
+      // one 128-byte-wide box covers the whole head
+      if (lane < 8) {
+        if (do_k) tma_load_2d(smem + L::kK + s * L::kRawStage + pg * (kPage * 128), &tmK, &k_full[s], kvh * kD, blk * kPage);
+        if (do_v) tma_load_2d(smem + L::kV + s * L::kRawStage + pg * (kPage * 128), &tmV, &v_full[s], kvh * kD, blk * kPage);
       }
       __syncwarp();
     }
@@ -339,22 +192,20 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     // ---- Q tile -> shared, swizzled operand layout (slabs of 64 head elements); fp16 for e4m3 pages.  The
     // two producer warps are already fetching K and V meanwhile; the MMA issuer waits for q_ready. ----
     const int st = (warp == 1 ? 0 : warp - 2) * 32 + lane;       // 0..575
-    for (int c = st; c < kRows * 8 * KS; c += 18 * 32) {
-      const int row = c / (8 * KS), ch = c % (8 * KS);
+    for (int c = st; c < kRows * 16; c += 18 * 32) {
+      const int row = c / 16, ch = c % 16;
       uint4 v = make_uint4(0, 0, 0, 0);
       if (row_base + row < n)
-        v = *reinterpret_cast<const uint4*>(p.q + (static_cast<size_t>(q_begin + row_base + row) * p.Hq + h) * (64 * KS) + ch * 8);
-      if (FP8) {
-        const __nv_bfloat162* bv = reinterpret_cast<const __nv_bfloat162*>(&v);
-        uint32_t o[4];
+        v = *reinterpret_cast<const uint4*>(p.q + (static_cast<size_t>(q_begin + row_base + row) * p.Hq + h) * kD + ch * 8);
+      const __nv_bfloat162* bv = reinterpret_cast<const __nv_bfloat162*>(&v);
+      uint32_t o[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 f = __bfloat1622float2(bv[i]);
-          const __half2 hh = __floats2half2_rn(f.x, f.y);
-          o[i] = *reinterpret_cast<const uint32_t*>(&hh);
-        }
-        v = make_uint4(o[0], o[1], o[2], o[3]);
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(bv[i]);
+        const __half2 hh = __floats2half2_rn(f.x, f.y);
+        o[i] = *reinterpret_cast<const uint32_t*>(&hh);
       }
+      v = make_uint4(o[0], o[1], o[2], o[3]);
       *reinterpret_cast<uint4*>(smem + L::kQ + (ch >> 3) * kSlab + swz_chunk(row, ch & 7)) = v;
     }
     fence_proxy_async();
@@ -366,8 +217,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
-      constexpr uint32_t id_qk = idesc16(FP8 ? 0u : 1u, false);
-      constexpr uint32_t id_pv = idesc16(FP8 ? 0u : 1u, true);
+      constexpr uint32_t id_qk = idesc16(0u, false);
+      constexpr uint32_t id_pv = idesc16(0u, true);
       const uint32_t q_addr = smem_u32(smem + L::kQ);
       const uint32_t p_base = smem_u32(smem + L::kP);
       bool ok = true;
@@ -375,36 +226,26 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         const int s = j & 1;
         if (j >= 2 && !mbar_wait(&s_free[s], ((j >> 1) - 1) & 1)) { report(p.status, kErrMmaWaitAccum); return false; }
         uint32_t k_addr;
-        if (FP8) {
-          if (!mbar_wait(kc_ready, j & 1)) { report(p.status, kErrMmaWaitFull); return false; }
-          k_addr = smem_u32(smem + L::kK + 2 * L::kRawStage);
-        } else {
-          if (!mbar_wait(&k_full[s], (j >> 1) & 1)) { report(p.status, kErrMmaWaitFull); return false; }
-          k_addr = smem_u32(smem + L::kK + s * L::kKTile);
-        }
+        if (!mbar_wait(kc_ready, j & 1)) { report(p.status, kErrMmaWaitFull); return false; }
+        k_addr = smem_u32(smem + L::kK + 2 * L::kRawStage);
         tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < 4 * KS; ++k) { // 16 head elements (32 bytes) per MMA; 4 per slab
+        for (int k = 0; k < 8; ++k) { // 16 head elements (32 bytes) per MMA; 4 per slab
           const uint64_t da = make_desc_sw128(q_addr + (k >> 2) * kSlab) + ((k & 3) * 32 >> 4);
           const uint64_t db = make_desc_sw128(k_addr + (k >> 2) * kSlab) + ((k & 3) * 32 >> 4);
           mma_f16(tS + s * 128, da, db, id_qk, k > 0 ? 1u : 0u);
         }
         tc_commit(&s_full[s]);
-        tc_commit(FP8 ? kc_free : &k_free[s]);
+        tc_commit(kc_free);
         return true;
       };
       auto issue_pv = [&](int j) {
-        const int s = j & 1, vs = L::stage(j);
+        const int s = j & 1, vs = s;
         if (j >= 2 && !mbar_wait(&pv_free[s], ((j >> 1) - 1) & 1)) { report(p.status, kErrMmaWaitAccum); return false; }
         uint32_t v_addr;
-        if (FP8) {
-          if (!mbar_wait(vc_ready, j & 1)) { report(p.status, kErrMmaWaitFull); return false; }
-          v_addr = smem_u32(smem + L::kV + 2 * L::kRawStage);
-        } else {
-          if (!mbar_wait(&v_full[vs], L::round(j) & 1)) { report(p.status, kErrMmaWaitFull); return false; }
-          v_addr = smem_u32(smem + L::kV + vs * kTileBytes);
-        }
-        if (!mbar_wait(&p_ready[vs], L::round(j) & 1)) { report(p.status, kErrMmaWaitFull); return false; }
+        if (!mbar_wait(vc_ready, j & 1)) { report(p.status, kErrMmaWaitFull); return false; }
+        v_addr = smem_u32(smem + L::kV + 2 * L::kRawStage);
+        if (!mbar_wait(&p_ready[vs], (j >> 1) & 1)) { report(p.status, kErrMmaWaitFull); return false; }
         const uint32_t p_addr = p_base + vs * kTileBytes;
         tc_fence_after();
 #pragma unroll
@@ -415,7 +256,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         }
         tc_commit(&pv_full[s]);
         tc_commit(&p_free[vs]);
-        tc_commit(FP8 ? vc_free : &v_free[vs]);
+        tc_commit(vc_free);
         return true;
       };
       ok = mbar_wait(q_ready, 0);
@@ -438,7 +279,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     const int pos = pos_first + r;
     int hz = pos;
     if (p.horizon != nullptr && row_base + r < n) hz = max(pos, min(p.horizon[q_begin + row_base + r], Lkv - 1));
-    const float ks = (FP8 && p.k_scale != nullptr) ? p.k_scale[kvh] : 1.f;
+    const float ks = p.k_scale != nullptr ? p.k_scale[kvh] : 1.f;
     const float raw_scale = p.scale * ks;
     const float scale_log2 = raw_scale * kLog2e;
     const uint32_t lane_addr = tS + (static_cast<uint32_t>(quarter * 32) << 16) + hf * 64;
@@ -455,7 +296,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     // barrier; everyone reads the flag right after the barrier, where all 64 threads see the same value.
     bool fail = false;
     for (int j = 0; j < ntiles; ++j) {
-      const int s = j & 1, ps = L::stage(j);
+      const int s = j & 1, ps = s;
       const int t0 = tile_start(j) + hf * 64;       // first key of this thread's half
       const int t_min = j < kept ? 0 : win_min, t_max = j < kept ? min(p.keep, win_min) - 1 : win_max;
       if (!fail && !mbar_wait(&s_full[s], (j >> 1) & 1)) { report(p.status, kErrEpilogueWait); fail = true; }
@@ -487,7 +328,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
       const float m_new = fmaxf(m, fmaxf(mx, s_rowmax[(hf ^ 1) * 128 + r]));
       const float alpha = m_new == -INFINITY ? 0.f : fast_exp2(m - m_new);
       // the P tile and this parity's alpha slot are free once the PV product two tiles back was consumed
-      if (j >= L::kStagesVP && !mbar_wait(&p_free[ps], (L::round(j) - 1) & 1)) { report(p.status, kErrEpilogueWait); fail = true; }
+      if (j >= 2 && !mbar_wait(&p_free[ps], ((j >> 1) - 1) & 1)) { report(p.status, kErrEpilogueWait); fail = true; }
       if (!fail && j >= 2 && !mbar_wait(&pv_free[s], ((j >> 1) - 1) & 1)) { report(p.status, kErrEpilogueWait); fail = true; }
       if (fail) continue;
       // pass 2: probabilities as 16-bit values into the P operand tile, partial row sum.  A row without a visible
@@ -498,10 +339,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         if (c == 0) tmem_ld32(lane_addr + s * 128, v);
         uint32_t packed[16];
         sa.lo = t_max >= t_min ? t_min - (t0 + c) : (1 << 30);
-        if (plain && !cap) rs += group_prob<false, false, FP8>(v, packed, m_new, sa);
-        else if (!cap) rs += group_prob<true, false, FP8>(v, packed, m_new, sa);
-        else if (plain) rs += group_prob<false, true, FP8>(v, packed, m_new, sa);
-        else rs += group_prob<true, true, FP8>(v, packed, m_new, sa);
+        if (plain && !cap) rs += group_prob<false, false, true, kPolyEvery>(v, packed, m_new, sa);
+        else if (!cap) rs += group_prob<true, false, true, kPolyEvery>(v, packed, m_new, sa);
+        else if (plain) rs += group_prob<false, true, true, kPolyEvery>(v, packed, m_new, sa);
+        else rs += group_prob<true, true, true, kPolyEvery>(v, packed, m_new, sa);
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {      // four 16-byte chunks (8 keys each) of this 32-key group
           const int ch = hf * 8 + (c >> 3) + q4;   // chunk index among the row's 16
@@ -522,13 +363,13 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     }
     // partial row sums into the P tile the last product does not read; that tile was last read by the product of
     // the tile before the last one
-    if (!fail && L::kStagesVP == 2 && ntiles >= 2 && !mbar_wait(&p_free[ntiles & 1], ((ntiles - 2) >> 1) & 1)) {
+    if (!fail && ntiles >= 2 && !mbar_wait(&p_free[ntiles & 1], ((ntiles - 2) >> 1) & 1)) {
       report(p.status, kErrEpilogueWait);
       fail = true;
     }
     if (!fail) {
       if (p.sink != nullptr && hf == 0) l += exp2f(fmaf(p.sink[h], kLog2e, -m));      // both threads of a row hold the same maximum
-      reinterpret_cast<float*>(smem + (L::kStagesVP == 2 ? L::kP + (ntiles & 1) * kTileBytes : L::kSums))[hf * 128 + r] = l;
+      reinterpret_cast<float*>(smem + L::kP + (ntiles & 1) * kTileBytes)[hf * 128 + r] = l;
       __syncwarp();
       if (lane == 0) mbar_arrive(l_ready);
     }
@@ -576,14 +417,12 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
       }
       return true;
     };
-    if (FP8) {
-      ok = convert(0, 0);
-      if (ok && ntiles > 1) ok = convert(0, 1);
-      if (ok) ok = convert(1, 0);
-    }
+    ok = convert(0, 0);
+    if (ok && ntiles > 1) ok = convert(0, 1);
+    if (ok) ok = convert(1, 0);
     for (int j = 0; j < ntiles && ok; ++j) {
       const int s = j & 1;
-      if (FP8 && j + 2 < ntiles && !convert(0, j + 2)) { ok = false; break; }
+      if (j + 2 < ntiles && !convert(0, j + 2)) { ok = false; break; }
       if (!mbar_wait(&pv_full[s], (j >> 1) & 1)) { report(p.status, kErrEpilogueWait); ok = false; break; }
       tc_fence_after();
       const float alpha = s_alpha[s * 128 + r];
@@ -598,11 +437,11 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&pv_free[s]);
-      if (FP8 && j + 1 < ntiles && !convert(1, j + 1)) { ok = false; break; }
+      if (j + 1 < ntiles && !convert(1, j + 1)) { ok = false; break; }
     }
     if (ok && mbar_wait(l_ready, 0)) {
-      const float vs = (FP8 && p.v_scale != nullptr) ? p.v_scale[kvh] : 1.f;
-      const float* s_rowsum = reinterpret_cast<const float*>(smem + (L::kStagesVP == 2 ? L::kP + (ntiles & 1) * kTileBytes : L::kSums));
+      const float vs = p.v_scale != nullptr ? p.v_scale[kvh] : 1.f;
+      const float* s_rowsum = reinterpret_cast<const float*>(smem + L::kP + (ntiles & 1) * kTileBytes);
       const float l = s_rowsum[r] + s_rowsum[128 + r];
       float inv = l > 0.f ? vs / l : 0.f;
       if (p.gate != nullptr && row_base + r < n)
@@ -626,26 +465,17 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
   if (warp == 1) tmem_dealloc(tmem_base, 512);
 }
 
-// `k_pitch`, `v_pitch`: elements from a token's keys (values) to the next token's
-template <bool FP8, int KS>
 int launch_prefill(const PrefillParams& p, const void* k_cache, const void* v_cache, long long k_pitch, long long v_pitch, int B,
                    int max_q, cudaStream_t stream) {
-  using L = Layout<FP8, KS>;
+  using L = Layout;
   CUtensorMap tmK, tmV;
   const uint64_t rows = static_cast<uint64_t>(p.num_blocks) * kPage;
-  const uint64_t k_cols = static_cast<uint64_t>(p.Hkv) * 64 * KS, v_cols = static_cast<uint64_t>(p.Hkv) * kD;
-  int rc;
-  if (FP8) {
-    rc = tgi::make_map_2d(&tmK, CU_TENSOR_MAP_DATA_TYPE_UINT8, k_cache, rows, k_cols, k_pitch, kPage, 128, CU_TENSOR_MAP_SWIZZLE_NONE);
-    if (rc) return rc;
-    rc = tgi::make_map_2d(&tmV, CU_TENSOR_MAP_DATA_TYPE_UINT8, v_cache, rows, v_cols, v_pitch, kPage, 128, CU_TENSOR_MAP_SWIZZLE_NONE);
-  } else {
-    rc = tgi::make_map_2d(&tmK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, k_cache, rows, k_cols, k_pitch * 2, kPage, 64, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc) return rc;
-    rc = tgi::make_map_2d(&tmV, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, v_cache, rows, v_cols, v_pitch * 2, kPage, 64, CU_TENSOR_MAP_SWIZZLE_128B);
-  }
+  const uint64_t k_cols = static_cast<uint64_t>(p.Hkv) * kD, v_cols = k_cols;
+  int rc = tgi::make_map_2d(&tmK, CU_TENSOR_MAP_DATA_TYPE_UINT8, k_cache, rows, k_cols, k_pitch, kPage, 128, CU_TENSOR_MAP_SWIZZLE_NONE);
   if (rc) return rc;
-  auto kern = prefill_tc_kernel<FP8, KS>;
+  rc = tgi::make_map_2d(&tmV, CU_TENSOR_MAP_DATA_TYPE_UINT8, v_cache, rows, v_cols, v_pitch, kPage, 128, CU_TENSOR_MAP_SWIZZLE_NONE);
+  if (rc) return rc;
+  auto kern = prefill_e4m3_kernel;
   static std::atomic<unsigned long long> attr_set{0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return -2;
@@ -660,6 +490,11 @@ int launch_prefill(const PrefillParams& p, const void* k_cache, const void* v_ca
 }
 
 }  // namespace
+
+int prefill::launch_e4m3(const PrefillParams& p, const void* k_cache, const void* v_cache, long long k_pitch, long long v_pitch, int B,
+                         int max_q, cudaStream_t stream) {
+  return launch_prefill(p, k_cache, v_cache, k_pitch, v_pitch, B, max_q, stream);
+}
 
 extern "C" {
 
@@ -693,8 +528,8 @@ int tgi_prefill_attention_tc(const void* q, const void* k_cache, const void* v_c
   p.sink = sink;
   p.status = status;
   const long long pitch = static_cast<long long>(Hkv) * kD;
-  return fp8_kv ? launch_prefill<true, 2>(p, k_cache, v_cache, pitch, pitch, B, max_q, stream)
-                : launch_prefill<false, 2>(p, k_cache, v_cache, pitch, pitch, B, max_q, stream);
+  return fp8_kv ? prefill::launch_e4m3(p, k_cache, v_cache, pitch, pitch, B, max_q, stream)
+                : prefill::launch_bf16(p, kD, k_cache, v_cache, pitch, pitch, B, max_q, stream);
 }
 
 // The same on keys and values of H heads that were written out for this step: q [T, H, dim] bf16 with dim 128 or 192, a
@@ -722,8 +557,7 @@ int tgi_expanded_attention(const void* q, const void* k, const void* v, long lon
   p.window = window;
   p.sink = sink;
   p.status = status;
-  return dim == 192 ? launch_prefill<false, 3>(p, k, v, pitch, pitch, B, max_q, stream)
-                    : launch_prefill<false, 2>(p, k, v, pitch, pitch, B, max_q, stream);
+  return prefill::launch_bf16(p, dim, k, v, pitch, pitch, B, max_q, stream);
 }
 
 }  // extern "C"
