@@ -37,8 +37,8 @@
 // partial tile and counts its arrival; after its own main loop each contributor waits (bounded)
 // for the others and reduces its own slice of the tile's columns, summing the partials in CTA
 // order, so the work of the fix-up is spread over the contributors and the result does not depend
-// on arrival order.  Problems with fewer tiles than SMs use whole tiles or a few aligned K splits
-// instead when that is cheaper (see launch()).
+// on arrival order.  Where it is cheaper (see launch()) the shares start on tiles, in rounds, and
+// problems with fewer tiles than SMs use whole tiles or a few aligned K splits.
 //
 // Roles inside a CTA (384 threads): warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner
 // (warps 2, 3 idle; the four give their registers away with setmaxnreg), warps 4..11 = promotion /
@@ -152,8 +152,12 @@ struct AccPairs {
 
 struct Sched {
   int n_tiles, m_tiles, KB, grid;
+  int whole_tiles;           // ranges start on tiles
   long long units;
-  __device__ __forceinline__ long long begin(int c) const { return units * c / grid; }
+  __device__ __forceinline__ long long begin(int c) const {
+    if (whole_tiles) return static_cast<long long>(n_tiles) * m_tiles * c / grid * KB;
+    return units * c / grid;
+  }
   __device__ __forceinline__ int owner(long long u) const {   // CTA whose range contains unit u
     int c = static_cast<int>(u * grid / units);
     while (c + 1 < grid && begin(c + 1) <= u) ++c;
@@ -199,7 +203,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                     const __grid_constant__ CUtensorMap tmS, const float* __restrict__ wscale,
                     __nv_bfloat16* __restrict__ C, const __nv_bfloat16* __restrict__ bias, int M, int N, int K,
-                    float* __restrict__ ws, int* __restrict__ counters, int* __restrict__ status,
+                    float* __restrict__ ws, int* __restrict__ counters, int* __restrict__ status, int whole_tiles,
                     const __grid_constant__ PushArgs push) {
   using Cfg = TileCfg<MH, TN, PAIR, FP8, MX>;
   static_assert(!MX || FP8, "the block-scaled mode is built for fp8 operands");
@@ -252,6 +256,7 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   sch.n_tiles = (N + TN - 1) / TN;
   sch.m_tiles = (M + TM - 1) / TM;
   sch.KB = (K + BK - 1) / BK;
+  sch.whole_tiles = whole_tiles;
   sch.grid = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
   sch.units = static_cast<long long>(sch.n_tiles) * sch.m_tiles * sch.KB;
   const long long u0 = sch.begin(worker), u1 = sch.begin(worker + 1);
@@ -584,9 +589,11 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
         const int first_tile = static_cast<int>(u0 / sch.KB);
         const int slot = blockIdx.x * 2 + (tile == first_tile ? 0 : 1);
         float4* wsp = reinterpret_cast<float4*>(ws + static_cast<size_t>(slot) * kTileElems) + et;
+        if (warp_active) {
 #pragma unroll
-        for (int j = 0; j < kCols; j += 4)
-          wsp[(j >> 2) * kEpiThreads] = make_float4(acc.get(j), acc.get(j + 1), acc.get(j + 2), acc.get(j + 3));
+          for (int j = 0; j < kCols; j += 4)
+            wsp[(j >> 2) * kEpiThreads] = make_float4(acc.get(j), acc.get(j + 1), acc.get(j + 2), acc.get(j + 3));
+        }
         __threadfence();
         epi_barrier();
         if (et == 0) atomicAdd(&counters[counter_of(tile)], 1);
@@ -653,18 +660,32 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
       const int m = m0 + m_local;
       const int nb = n0 + n_off;
       const float4* wsb = reinterpret_cast<const float4*>(ws) + et;
-      for (int jc = jc0; jc < jc1; ++jc) {
-        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+      // kBatch columns at a time, so that a batch's loads are under way together: a thread has 32 of them
+      constexpr int kBatch = 8;
+      for (int jb = jc0; jb < jc1; jb += kBatch) {
+        if (m >= M || nb >= N) break;
+        float4 sum[kBatch];
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q) sum[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
         for (int i = 0; i < n; ++i) {
-          const float4 t = __ldcg(wsb + static_cast<size_t>(cslots[i]) * (kTileElems / 4) + jc * kEpiThreads);
-          sum.x += t.x;
-          sum.y += t.y;
-          sum.z += t.z;
-          sum.w += t.w;
+          const float4* src = wsb + static_cast<size_t>(cslots[i]) * (kTileElems / 4) + jb * kEpiThreads;
+          float4 t[kBatch];
+#pragma unroll
+          for (int q = 0; q < kBatch; ++q) t[q] = jb + q < jc1 ? __ldcg(src + q * kEpiThreads) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int q = 0; q < kBatch; ++q) {
+            sum[q].x += t[q].x;
+            sum[q].y += t[q].y;
+            sum[q].z += t[q].z;
+            sum[q].w += t[q].w;
+          }
         }
-        const int col = nb + jc * 4;
-        if (m < M && col < N) {
-          float f[4] = {sum.x, sum.y, sum.z, sum.w};
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q) {
+          const int col = nb + (jb + q) * 4;
+          if (jb + q >= jc1 || col >= N) continue;
+          float f[4] = {sum[q].x, sum[q].y, sum[q].z, sum[q].w};
           if (bias != nullptr) {
 #pragma unroll
             for (int e = 0; e < 4; ++e)
@@ -804,6 +825,20 @@ int launch(const void* X, const float* xs_t, int xs_pitch, const void* W, const 
   int grid = max_workers;
   if (grid > units) grid = static_cast<int>(units);
   if (grid < 1) grid = 1;
+  int whole_tiles = 0;
+  if (tiles > max_workers && !(FP8 && M > Cfg::TM)) {
+    // Whole tiles in rounds, or equal shares whose cut tiles are put together through global memory.  On B200 the latter costs
+    // about 34 us whatever the sizes, a K block about 0.5 us.  Equal shares / whole tiles in us: 28672 x 4096 bf16 (112 pair tiles on
+    // 74 pairs) with 201 tokens 76 / 56, 128256 x 4096 with 201 237 / 215 and with 64 195 / 164, 57344 x 8192 fp8 with 64 104 / 84,
+    // with 256 143 / 136.  Prompts in fp8 (several token tiles) keep equal shares: there the two are equally fast (3300 tokens of
+    // a 70B model 34 / 34 ms), and a model that quantises its activations anew for every product would change its results.
+    const int rounds = (tiles + max_workers - 1) / max_workers;
+    const long long extra = static_cast<long long>(rounds) * KBn - (units + max_workers - 1) / max_workers;
+    if (extra * 0.5 < 34.0) {
+      whole_tiles = 1;
+      grid = (tiles + rounds - 1) / rounds;
+    }
+  }
   if (tiles <= max_workers) {
     // Rough costs in microseconds, from timelines measured on B200: a K block takes about 0.4 us per
     // CTA; every partial tile costs 128 KB written and read through L2 by all CTAs at once (about
@@ -827,7 +862,7 @@ int launch(const void* X, const float* xs_t, int xs_pitch, const void* W, const 
   const cudaError_t err =
       tgi::launch_cluster(kern, dim3(PAIR ? 2 * grid : grid), dim3(kThreads), smem, stream, PAIR ? 2 : 1, tmW, tmX, tmS,
                           wscale, static_cast<__nv_bfloat16*>(C), static_cast<const __nv_bfloat16*>(bias), M, N, K, ws,
-                          counters, status, push);
+                          counters, status, whole_tiles, push);
   return err == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
