@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                     const __grid_constant__ CUtensorMap tmS, const float* __restrict__ wscale,
                     __nv_bfloat16* __restrict__ C, const __nv_bfloat16* __restrict__ bias, int M, int N, int K,
-                    float* __restrict__ ws, int* __restrict__ counters, int* __restrict__ status, int whole_tiles,
+                    float* __restrict__ ws, int* __restrict__ counters, int* __restrict__ status, int whole_tiles, int settled,
                     const __grid_constant__ PushArgs push) {
   using Cfg = TileCfg<MH, TN, PAIR, FP8, MX>;
   static_assert(!MX || FP8, "the block-scaled mode is built for fp8 operands");
@@ -303,8 +303,10 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   const uint32_t tmem_empty0_remote = PAIR ? map_to_cta(smem_u32(&tmem_empty[0]), 0) : 0u;
   const uint32_t sf_ready0_remote = (PAIR && MX) ? map_to_cta(smem_u32(&sf_ready[0]), 0) : 0u;
   // Barrier set-up, TMEM allocation and descriptor prefetch above touch no tensor data, so they overlap
-  // with the tail of the previous kernel; from here on the operands (and the workspace) are used.
-  tgi::pdl_wait();
+  // with the tail of the previous kernel; from here on the operands (and the workspace) are used.  Settled weights
+  // (gemm_skinny.h) fill the ring before that: the producer waits behind them.  Decode steps: 8B 201 sequences 5404 -> 5323 us,
+  // 70B fp8 256 sequences 4350 -> 4269, Mixtral 48 sequences 2435 -> 2389.
+  if (warp != 0 || !settled) tgi::pdl_wait();
   tgi::pdl_trigger();
 
   if (warp < 4) {
@@ -316,6 +318,25 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
         const uint64_t pol_x = policy_evict_last();    // token tiles are re-read by every weight slab
         int issued = 0;
         bool ok = true;
+        constexpr uint32_t kCtaBytes = Cfg::kStageBytes + (PROMOTE ? CM * 4 : 0);
+        auto load_weights = [&](int s, int kb, int n0) {
+          uint8_t* dst = smem + s * Cfg::kStageBytes + Cfg::kXBytes;
+          if (PAIR) {
+            // both CTAs' bytes are counted on the leader's barrier; only the leader posts the expectation
+            if (crank == 0) mbar_arrive_expect_tx(&full[s], 2 * kCtaBytes);
+            tma_load_2d_pair_hint(dst, &tmW, full0_remote + s * 8, kb * BK, n0 + static_cast<int>(crank) * Cfg::WROWS, pol_w);
+          } else {
+            mbar_arrive_expect_tx(&full[s], kCtaBytes);
+#pragma unroll
+            for (int h = 0; h < TN / 128; ++h) tma_load_2d_hint(dst + h * 16384, &tmW, &full[s], kb * BK, n0 + h * 128, pol_w);
+          }
+        };
+        int ahead = 0;             // stages whose weights are already on their way
+        if (settled) {
+          UnitIter w(u0, sch);
+          for (; ahead < STAGES && ahead < nunits; ++ahead, w.next(sch)) load_weights(ahead, w.kb, w.tn * TN);
+          tgi::pdl_wait();
+        }
         UnitIter ui(u0, sch);
         for (int it = 0; it < nunits && ok; ++it, ui.next(sch)) {
           const int kb = ui.kb;
@@ -327,13 +348,10 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
           // MX: with a stage go the activation scales of the K block AFTER its own (with the first stage also its
           // own), on barriers of their own, so that a K block's scale factors are in TMEM before its operands land
           const bool sc_next = MX && it + 1 < nunits;
-          constexpr uint32_t kCtaBytes = Cfg::kStageBytes + (PROMOTE ? CM * 4 : 0);
+          if (it >= ahead) load_weights(s, kb, n0);
           if (PAIR) {
-            // both CTAs' bytes are counted on the leader's barrier; only the leader posts the expectation
             const uint32_t bar = full0_remote + s * 8;
-            if (crank == 0) mbar_arrive_expect_tx(&full[s], 2 * kCtaBytes);
             tma_load_2d_pair_hint(st, &tmX, bar, kb * BK, m0 + static_cast<int>(crank) * CM, pol_x);
-            tma_load_2d_pair_hint(st + Cfg::kXBytes, &tmW, bar, kb * BK, n0 + static_cast<int>(crank) * Cfg::WROWS, pol_w);
             if (PROMOTE) tma_load_2d_pair(sc_ring + (it % SC_STAGES) * CM, &tmS, bar, m0 + static_cast<int>(crank) * CM, kb);
             if (MX) {      // every CTA fetches the scales of its own token rows, on its own barriers
               if (it == 0) {
@@ -349,12 +367,8 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
               }
             }
           } else {
-            mbar_arrive_expect_tx(&full[s], kCtaBytes);
 #pragma unroll
             for (int h = 0; h < MH; ++h) tma_load_2d_hint(st + h * 16384, &tmX, &full[s], kb * BK, m0 + h * 128, pol_x);
-#pragma unroll
-            for (int h = 0; h < TN / 128; ++h)
-              tma_load_2d_hint(st + Cfg::kXBytes + h * 16384, &tmW, &full[s], kb * BK, n0 + h * 128, pol_w);
             if (PROMOTE) tma_load_2d(sc_ring + (it % SC_STAGES) * TM, &tmS, &full[s], m0, kb);
             if (MX) {
               if (it == 0) {
@@ -747,7 +761,7 @@ int g_streamk_small = 0;   // 1: problems with fewer tiles than workers may also
 
 template <int MH, int TN, int STAGES, bool FP8, bool PAIR, bool MX = false>
 int launch(const void* X, const float* xs_t, int xs_pitch, const void* W, const float* wscale, void* C,
-           const void* bias, int M, int N, int K, int ldx, int max_ctas, float* ws, int* counters, int* status,
+           const void* bias, int M, int N, int K, int ldx, int max_ctas, int settled, float* ws, int* counters, int* status,
            cudaStream_t stream, const PushArgs* push_args = nullptr) {
   using Cfg = TileCfg<MH, TN, PAIR, FP8, MX>;
   PushArgs push;
@@ -860,9 +874,9 @@ int launch(const void* X, const float* xs_t, int xs_pitch, const void* W, const 
   }
   g_last_grid = PAIR ? 2 * grid : grid;
   const cudaError_t err =
-      tgi::launch_cluster(kern, dim3(PAIR ? 2 * grid : grid), dim3(kThreads), smem, stream, PAIR ? 2 : 1, tmW, tmX, tmS,
+      tgi::launch_cluster_after(settled || tgi::pdl_enabled(), kern, dim3(PAIR ? 2 * grid : grid), dim3(kThreads), smem, stream, PAIR ? 2 : 1, tmW, tmX, tmS,
                           wscale, static_cast<__nv_bfloat16*>(C), static_cast<const __nv_bfloat16*>(bias), M, N, K, ws,
-                          counters, status, whole_tiles, push);
+                          counters, status, whole_tiles, settled, push);
   return err == cudaSuccess && cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -893,11 +907,11 @@ static int g_mx_pairs = 1;        // CTA pairs in the block-scaled mode
 namespace {
 template <bool FP8>
 int dispatch(const void* X, const float* xs_t, int xs_pitch, const void* W, const float* wscale, void* C, const void* bias,
-             int M, int N, int K, int ldx, int max_ctas, float* ws, int* counters, int* status, cudaStream_t stream,
+             int M, int N, int K, int ldx, int max_ctas, int settled, float* ws, int* counters, int* status, cudaStream_t stream,
              const PushArgs* push) {
   if (FP8 && g_fp8_mx) {
     if (M <= g_wide_m)
-      return launch<1, 256, 4, FP8, false, FP8>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, ldx, max_ctas, ws, counters,
+      return launch<1, 256, 4, FP8, false, FP8>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, ldx, max_ctas, settled, ws, counters,
                                                  status, stream, push);
     const long long mx_pair_tiles = static_cast<long long>((N + 255) / 256) * ((M + 255) / 256);
     // pairs need enough work to repay their fixed cost: 256 x 8192 x 4096 (32 tiles of 32 K blocks) takes 30.7 us in
@@ -906,26 +920,26 @@ int dispatch(const void* X, const float* xs_t, int xs_pitch, const void* W, cons
     const long long mx_pair_units = mx_pair_tiles * ((K + 127) / 128);
     if (g_pairs && g_mx_pairs && max_ctas >= 2 && mx_pair_tiles >= g_pair_min_tiles &&
         (mx_pair_units >= 2048 || g_pair_min_tiles < 32)) {
-      const int rc = launch<1, 256, 6, FP8, FP8, FP8>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, ldx, max_ctas, ws, counters,
+      const int rc = launch<1, 256, 6, FP8, FP8, FP8>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, ldx, max_ctas, settled, ws, counters,
                                                        status, stream, push);
       if (rc != -4) return rc;
     }
-    return launch<2, 128, 4, FP8, false, FP8>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, ldx, max_ctas, ws, counters, status,
+    return launch<2, 128, 4, FP8, false, FP8>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, ldx, max_ctas, settled, ws, counters, status,
                                                stream, push);
   }
   if (M <= g_wide_m)
-    return launch<1, 256, 4, FP8, false>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, ldx, max_ctas, ws, counters, status,
+    return launch<1, 256, 4, FP8, false>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, ldx, max_ctas, settled, ws, counters, status,
                                          stream, push);
   // Pairs pay off when there are enough 256 x 256 tiles to go round: with few tiles (tensor-parallel shards, narrow
   // projections) the 74 pairs split K deeper than 148 single CTAs on 256 x 128 tiles do, and the fix-up of split
   // tiles costs more than the saved operand traffic (measured: 256 x 7168 x 8192 51 us in pairs, 48 us without).
   const long long pair_tiles = static_cast<long long>((N + 255) / 256) * ((M + 255) / 256);
   if (g_pairs && max_ctas >= 2 && pair_tiles >= g_pair_min_tiles) {
-    const int rc = launch<1, 256, 6, FP8, true>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, ldx, max_ctas, ws, counters,
+    const int rc = launch<1, 256, 6, FP8, true>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, ldx, max_ctas, settled, ws, counters,
                                                 status, stream, push);
     if (rc != -4) return rc;   // -4: this device cannot place a pair; fall back to single CTAs
   }
-  return launch<2, 128, 4, FP8, false>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, ldx, max_ctas, ws, counters, status,
+  return launch<2, 128, 4, FP8, false>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, ldx, max_ctas, settled, ws, counters, status,
                                        stream, push);
 }
 }  // namespace
@@ -965,7 +979,7 @@ int tgi_gemm_bf16(const void* X, const void* W, void* C, const void* bias, int M
   if (K % 8 != 0) return -10;  // TMA row pitch must be a multiple of 16 bytes
   if (tgi::skinny_bf16_applies(X, W, M, N, K, K, max_ctas))
     return tgi::skinny_bf16(X, K, W, C, bias, M, N, K, max_ctas, 0, status, stream);
-  return dispatch<false>(X, nullptr, 0, W, nullptr, C, bias, M, N, K, K, max_ctas, ws, counters, status, stream, nullptr);
+  return dispatch<false>(X, nullptr, 0, W, nullptr, C, bias, M, N, K, K, max_ctas, 0, ws, counters, status, stream, nullptr);
 }
 
 // The same with rows of X `ldx` elements apart (X may be a column slice of a wider matrix, 16-byte aligned).  settled: W and bias
@@ -976,7 +990,7 @@ int tgi_gemm_bf16_ld(const void* X, int ldx, const void* W, void* C, const void*
   if (K % 8 != 0 || ldx % 8 != 0 || ldx < K) return -10;
   if (tgi::skinny_bf16_applies(X, W, M, N, K, ldx, max_ctas))
     return tgi::skinny_bf16(X, ldx, W, C, bias, M, N, K, max_ctas, settled, status, stream);
-  return dispatch<false>(X, nullptr, 0, W, nullptr, C, bias, M, N, K, ldx, max_ctas, ws, counters, status, stream, nullptr);
+  return dispatch<false>(X, nullptr, 0, W, nullptr, C, bias, M, N, K, ldx, max_ctas, settled, ws, counters, status, stream, nullptr);
 }
 
 int tgi_gemm_fp8_block(const void* X, const float* xs_t, int xs_pitch, const void* W, const float* wscale, void* C,
@@ -986,7 +1000,7 @@ int tgi_gemm_fp8_block(const void* X, const float* xs_t, int xs_pitch, const voi
   if (K % 128 != 0 || xs_pitch % 4 != 0) return -10;
   if (tgi::skinny_fp8_applies(X, xs_t, W, M, K))
     return tgi::skinny_fp8(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, max_ctas, settled, status, stream);
-  return dispatch<true>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, K, max_ctas, ws, counters, status, stream, nullptr);
+  return dispatch<true>(X, xs_t, xs_pitch, W, wscale, C, bias, M, N, K, K, max_ctas, settled, ws, counters, status, stream, nullptr);
 }
 
 // Row-parallel GEMMs of a tensor-parallel group: same products, but every output row is stored into the
@@ -1003,10 +1017,10 @@ int tgi_gemm_push(int fp8, const void* X, const float* xs_t, int xs_pitch, const
   if (rc) return rc;
   if (fp8) {
     if (K % 128 != 0 || xs_pitch % 4 != 0) return -10;
-    return dispatch<true>(X, xs_t, xs_pitch, W, wscale, nullptr, bias, M, N, K, K, max_ctas, ws, counters, status, stream, &p);
+    return dispatch<true>(X, xs_t, xs_pitch, W, wscale, nullptr, bias, M, N, K, K, max_ctas, 0, ws, counters, status, stream, &p);
   }
   if (K % 8 != 0) return -10;
-  return dispatch<false>(X, nullptr, 0, W, nullptr, nullptr, bias, M, N, K, K, max_ctas, ws, counters, status, stream, &p);
+  return dispatch<false>(X, nullptr, 0, W, nullptr, nullptr, bias, M, N, K, K, max_ctas, 0, ws, counters, status, stream, &p);
 }
 
 }  // extern "C"

@@ -29,7 +29,7 @@ __device__ __forceinline__ void pdl_trigger() {
 #endif
 }
 
-// The trigger of the short kernels that a GEMM of a few tokens follows (norm, activation, quantisation, decode attention): such a
+// The trigger of the short kernels that a decode step's GEMMs follow (norm, activation, quantisation, decode attention): such a
 // GEMM may be launched so that it fetches settled weights meanwhile (`launch_after`), and its CTAs take nothing that these
 // kernels' later CTAs need, since all of those have started when the trigger takes effect.  Comes after `pdl_wait()`, so that what
 // runs ahead of its own wait runs after everything but its direct predecessor.
@@ -66,9 +66,9 @@ inline cudaError_t launch(void (*kernel)(Params...), dim3 grid, dim3 block, size
   return launch_after(pdl_enabled(), kernel, grid, block, smem, stream, args...);
 }
 
-// Same, with an optional thread-block cluster of `cluster_x` CTAs along x (1 = no cluster attribute).
+// `launch_after` with an optional thread-block cluster of `cluster_x` CTAs along x (1 = no cluster attribute).
 template <typename... Params, typename... Args>
-inline cudaError_t launch_cluster(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+inline cudaError_t launch_cluster_after(bool early, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                   int cluster_x, Args... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
@@ -84,7 +84,7 @@ inline cudaError_t launch_cluster(void (*kernel)(Params...), dim3 grid, dim3 blo
     attr[n].val.clusterDim.z = 1;
     ++n;
   }
-  if (pdl_enabled()) {
+  if (early) {
     attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[n].val.programmaticStreamSerializationAllowed = 1;
     ++n;

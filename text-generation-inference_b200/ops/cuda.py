@@ -220,10 +220,10 @@ def _gemm_ctas(lib, st, M: int, N: int, max_ctas: Optional[int]) -> int:
     return ctas
 
 
-def _settled(settled: bool, tokens: int) -> c_int:
-    """Whether the few-token GEMMs may fetch weights ahead of the stream's order.  Only inside a captured step: there the
-    launch ahead is a kernel of the step, and steps don't write weights."""
-    return c_int(1 if settled and tokens <= 32 and torch.cuda.is_current_stream_capturing() else 0)
+def _settled(settled: bool) -> c_int:
+    """Whether a GEMM may fetch weights ahead of the stream's order.  Only inside a captured step: there the launch ahead is a
+    kernel of the step, and steps don't write weights."""
+    return c_int(1 if settled and torch.cuda.is_current_stream_capturing() else 0)
 
 
 def gemm_bf16(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, max_ctas: Optional[int] = None,
@@ -259,7 +259,7 @@ def gemm_bf16(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = N
         return out.reshape(*lead, N)
     st = state(x.device)
     ctas = _gemm_ctas(lib, st, M, N, max_ctas)
-    early = _settled(settled, M)
+    early = _settled(settled)
     if sliced or early.value:
         _check(lib.tgi_gemm_bf16_ld(_ptr(x2), c_int(x2.stride(0) if sliced else K), _ptr(w), _ptr(out), _ptr(bias), c_int(M),
                                     c_int(N), c_int(K), c_int(ctas), early, _ptr(st.ws), _ptr(st.counters), _ptr(st.status), _stream()),
@@ -302,7 +302,7 @@ def gemm_fp8_block(xq, xs, wq, ws, out_dtype=torch.bfloat16, bias=None, max_ctas
     if not ws.is_contiguous():
         ws = ws.contiguous()
     _check(lib.tgi_gemm_fp8_block(_ptr(xq), c_void_p(sptr), c_int(pitch), _ptr(wq), _ptr(ws), _ptr(out), _ptr(bias),
-                                  c_int(M), c_int(N), c_int(K), c_int(ctas), _settled(settled, M), _ptr(st.ws), _ptr(st.counters),
+                                  c_int(M), c_int(N), c_int(K), c_int(ctas), _settled(settled), _ptr(st.ws), _ptr(st.counters),
                                   _ptr(st.status), _stream()), "gemm_fp8_block")
     return out
 
@@ -914,7 +914,7 @@ def gemm_wq(x: torch.Tensor, wq: torch.Tensor, scale: torch.Tensor, zp: Optional
     xh = torch.empty(M, K, dtype=torch.float16, device=x.device)       # fp16 copy of the tokens, written by the call
     _check(lib.tgi_gemm_wq(c_int(bits), _ptr(x), _ptr(xh), _ptr(wq), _ptr(scale), _ptr(zp), c_int(group), _ptr(out),
                            _ptr(part), c_ll(part.numel()), _ptr(bias), c_int(M), c_int(N), c_int(K), c_int(st.sm_count),
-                           _settled(settled, M), _ptr(st.status), _stream()), "gemm_wq")
+                           _settled(settled), _ptr(st.status), _stream()), "gemm_wq")
     return out
 
 
