@@ -516,9 +516,10 @@ sample_kernel(const T* __restrict__ scores, long long row_stride, const float* _
 
   if (!cut_typ && !odd && m > -INFINITY && m < INFINITY) {
     // ---- second pass: the entries within kReach of the maximum ----
-    const float low = m - kReach;
+    // compared as order_bits, as the keys below are: these put -0 under +0
+    const uint32_t base = order_bits(m - kReach);
     auto put = [&](int i, float x) {
-      if (x >= low) {
+      if (order_bits(x) >= base) {
         const int at = atomicAdd(&s_n, 1);
         if (at < kList) {
           list_x[at] = x;
@@ -529,7 +530,6 @@ sample_kernel(const T* __restrict__ scores, long long row_stride, const float* _
     row.each(put);
     __syncthreads();
     const int n = s_n;
-    const uint32_t base = order_bits(low);
     const int bits = 32 - __clz(order_bits(m) - base);
     auto listed = [&](auto&& f) {
       for (int j = threadIdx.x; j < n; j += THREADS) f(list_i[j], list_x[j]);
