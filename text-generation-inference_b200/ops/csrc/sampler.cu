@@ -10,9 +10,9 @@
 //   keyed by the request's seed with counter (j, step): reproducible for a given seed.
 //   logprob = x_c - logsumexp over the kept set.
 //
-// What bounds it is reading the logits once from DRAM (256 rows x 128256 bf16: 66 MB, 10 us).  A row that nothing cuts
-// is read once: running maximum and sum, four noises from one Philox block.  A row that top-k or top-p cut is read
-// twice, the second time from L2 and only to collect the entries within kReach of the maximum; as a rule they decide
+// What bounds it is reading the logits once from DRAM (256 rows x 128256 bf16: 66 MB, 10 us).  A row is read for its maximum and,
+// from L2, once more: one that nothing cuts for its mass and the choice (four noises from one Philox block), one that top-k or
+// top-p cut for its mass (top-p alone) and to collect the entries within kReach of the maximum; as a rule they decide
 // both cuts (top-k: there are at least k of them; top-p: their mass reaches p of the whole), and thresholds, noise and
 // sums are then a matter of a few hundred entries in shared memory.  Rows for which they do not (flat distributions
 // under a p near 1, more than kList entries that close) and typical-p take thresholds from histograms over the whole row.
@@ -112,17 +112,6 @@ struct Row {
   }
 };
 
-__device__ __forceinline__ float block_sum(float v, float* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  float t = 0.f;
-  for (int w = 0; w < (blockDim.x >> 5); ++w) t += red[w];
-  return t;
-}
 __device__ __forceinline__ unsigned long long block_sum(unsigned long long v, unsigned long long* red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -143,8 +132,9 @@ constexpr float kFixedOne = 1099511627776.f;   // 2^40
 constexpr float kReach = 8.f;            // entries below the maximum by more than this are not listed
 constexpr int kList = 4096;              // listed entries
 
-// Weights are summed as 2^-40 fixed point in 64-bit integers, so the sums do not depend on the order in which atomics
-// land: the same row always yields the same threshold and the same log-probability.
+// Weights are summed as 2^-40 fixed point in 64-bit integers, every one of them: the sums do not depend on the order in which atomics
+// land or penalised ids were listed, nor on the number of threads or the row's alignment.  The same row always yields the same
+// thresholds and the same log-probability, whatever batch it is in.
 __device__ __forceinline__ unsigned long long mass_of(float x, float m) {
   return static_cast<unsigned long long>(__expf(x - m) * kFixedOne);
 }
@@ -308,39 +298,61 @@ __device__ uint32_t row_threshold(const Row<T>& row, uint32_t floor_bits, float 
                                            m, lim, hist, tot);
 }
 
+// Mass of the entries of a row from `keep_from` on; `none`: some of them has no mass (NaN, or an infinite maximum).
+template <typename T>
+__device__ unsigned long long kept_mass(const Row<T>& row, float m, uint32_t keep_from, unsigned long long* red, bool& none) {
+  unsigned long long w = 0ull;
+  bool odd = false;
+  row.each([&](int, float x) {
+    if (order_bits(x) < keep_from) return;
+    const float e = __expf(x - m);
+    if (e == e) w += static_cast<unsigned long long>(e * kFixedOne);
+    else odd = true;
+  });
+  none = __syncthreads_or(odd);
+  return block_sum(w, red);
+}
+
 // Typical-p (utils/logits_process.py:389-448): over the entries the earlier filters kept, with p_j their
 // renormalised probabilities and H their entropy, keep the entries with the smallest |-log p_j - H| whose mass
 // reaches `mass`.  Returns the largest kept deviation as float bits (deviations are >= 0, so their bit patterns
 // order like the values); found by bisection, no sort.
 template <typename T>
-__device__ uint32_t typical_threshold(const Row<T>& row, float m, uint32_t keep_from, float mass, float* red, float* log_z_out,
-                                      float* entropy_out) {
-  float z = 0.f;
+__device__ uint32_t typical_threshold(const Row<T>& row, float m, uint32_t keep_from, float mass, unsigned long long* red,
+                                      float* log_z_out, float* entropy_out) {
+  // H = log z + sum of exp(x - m) (m - x) / z, the sum in the same fixed point (no term above 1 / e)
+  unsigned long long w = 0ull, s = 0ull;
+  bool odd = false;
   row.each([&](int, float x) {
-    if (order_bits(x) >= keep_from && x != -INFINITY) z += __expf(x - m);
-  });
-  const float log_z = __logf(block_sum(z, red));
-  float h = 0.f;
-  row.each([&](int, float x) {
-    if (order_bits(x) >= keep_from && x != -INFINITY) {
-      const float lp = x - m - log_z;
-      h -= __expf(lp) * lp;
+    if (order_bits(x) < keep_from || x == -INFINITY) return;
+    const float e = __expf(x - m);
+    if (e == e) {
+      w += static_cast<unsigned long long>(e * kFixedOne);
+      s += static_cast<unsigned long long>(e * (m - x) * kFixedOne);
+    } else {
+      odd = true;
     }
   });
-  const float H = block_sum(h, red);
+  odd = __syncthreads_or(odd);
+  w = block_sum(w, red);
+  s = block_sum(s, red);
+  const float z = odd ? __uint_as_float(0x7fc00000u) : static_cast<float>(w) / kFixedOne;
+  const float log_z = __logf(z), H = log_z + static_cast<float>(s) / kFixedOne / z;
   *log_z_out = log_z;
   *entropy_out = H;
-  uint32_t lo = 0u, hi = 0x7f800000u;       // predicate "mass of deviations <= t reaches `mass`": true at +inf
+  if (odd) return 0x7f800000u;
+  const unsigned long long lim = static_cast<unsigned long long>(fmaxf(mass * z, 0.f) * kFixedOne);
+  uint32_t lo = 0u, hi = 0x7f800000u;       // predicate "mass of deviations <= t reaches `lim`": true at +inf
   while (lo < hi) {
     const uint32_t mid = lo + ((hi - lo) >> 1);
-    float acc = 0.f;
+    unsigned long long acc = 0ull;
     row.each([&](int, float x) {
       if (order_bits(x) >= keep_from && x != -INFINITY) {
         const float lp = x - m - log_z;
-        if (__float_as_uint(fabsf(-lp - H)) <= mid) acc += __expf(lp);
+        if (__float_as_uint(fabsf(-lp - H)) <= mid) acc += mass_of(x, m);
       }
     });
-    if (block_sum(acc, red) >= mass) hi = mid;
+    if (block_sum(acc, red) >= lim) hi = mid;
     else lo = mid + 1;
   }
   return lo;
@@ -377,7 +389,7 @@ sample_kernel(const T* __restrict__ scores, long long row_stride, const float* _
   float* pen_x = reinterpret_cast<float*>(list_i + kList);                       // [kPenalised], with rep only
   int* pen_i = reinterpret_cast<int*>(pen_x + kPenalised);                       // [kPenalised]
   uint32_t* marks = reinterpret_cast<uint32_t*>(pen_i + kPenalised);             // [V / 32, rounded up]
-  __shared__ float red[32], s_x[32], s_z[32];
+  __shared__ float red[32], s_x[32];
   __shared__ int s_i[32], s_n;
   __shared__ uint32_t s_lo_hi[2];
   __shared__ unsigned long long red64[32];
@@ -415,78 +427,23 @@ sample_kernel(const T* __restrict__ scores, long long row_stride, const float* _
   const uint64_t seed = seeds != nullptr ? static_cast<uint64_t>(seeds[b]) : 0ull;
   const uint32_t step = steps != nullptr ? static_cast<uint32_t>(steps[b]) : 0u;
   const bool cut_k = k > 0 && k < V, cut_p = p < 1.f, cut_typ = typ < 1.f;
-  const bool whole = !cut_k && !cut_p && !cut_typ;
 
-  // ---- first pass: maximum, sum of exp(x - max), and for whole rows the choice ----
-  float m = -INFINITY, z = 0.f;
+  // ---- first pass: maximum ----
+  float m = -INFINITY;
   bool odd = false;               // a NaN somewhere
-  Best best;
-  auto add = [&](float x) {
+  row.each([&](int, float x) {
+    m = fmaxf(m, x);
     odd |= x != x;
-    if (x > m) {
-      z *= __expf(m - x);         // m = -inf: z is 0
-      m = x;
-    }
-    if (x > -INFINITY) z += __expf(x - m);
-  };
-  row.scan([&](int i, const float(&x)[Row<T>::VEC]) {
-    float vm = x[0];
-#pragma unroll
-    for (int j = 0; j < Row<T>::VEC; ++j) {
-      vm = fmaxf(vm, x[j]);
-      odd |= x[j] != x[j];
-    }
-    if (vm > m) {
-      z *= __expf(m - vm);
-      m = vm;
-    }
-    if (m > -INFINITY) {
-#pragma unroll
-      for (int j = 0; j < Row<T>::VEC; ++j) z += __expf(x[j] - m);
-    }
-    if (whole) {
-      if (sample) {
-#pragma unroll
-        for (int q = 0; q < Row<T>::VEC; q += 4) {
-          // one Philox block holds the noise of four entries (the same numbers as gumbel_noise entry by entry)
-          const uint4 r = philox4x32(static_cast<uint32_t>(i + q) >> 2, step, static_cast<uint32_t>(seed),
-                                     static_cast<uint32_t>(seed >> 32));
-          const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (x[q + j] == -INFINITY) continue;
-            best.take(x[q + j] + tgi_sampling::gumbel_of(w[j]), x[q + j], i + q + j);
-          }
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < Row<T>::VEC; ++j)
-          if (x[j] != -INFINITY) best.take(x[j], x[j], i + j);
-      }
-    }
-  }, [&](int i, float x) {
-    add(x);
-    if (whole && x != -INFINITY) best.take(sample ? x + gumbel_noise(static_cast<uint32_t>(i), step, seed) : x, x, i);
   });
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float m2 = __shfl_xor_sync(0xffffffffu, m, o), z2 = __shfl_xor_sync(0xffffffffu, z, o);
-    const float mm = fmaxf(m, m2);
-    z = (m == -INFINITY ? 0.f : z * __expf(m - mm)) + (m2 == -INFINITY ? 0.f : z2 * __expf(m2 - mm));
-    m = mm;
-  }
-  if (lane == 0) {
-    red[warp] = m;
-    s_z[warp] = z;
-  }
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane == 0) red[warp] = m;
   if (threadIdx.x == 0) s_n = 0;
   odd = __syncthreads_or(odd);
   m = red[0];
   for (int w = 1; w < kWarps; ++w) m = fmaxf(m, red[w]);
-  z = 0.f;
-  for (int w = 0; w < kWarps; ++w)
-    if (red[w] != -INFINITY) z += s_z[w] * __expf(red[w] - m);
   __syncthreads();
+  Best best;
 
   // the choice among `best` of all threads, and its log-probability
   auto finish = [&](float z_kept) {
@@ -509,13 +466,43 @@ sample_kernel(const T* __restrict__ scores, long long row_stride, const float* _
       logprob[b] = best.x - m - __logf(z_kept);
     }
   };
-  if (whole) {
-    finish(odd ? __uint_as_float(0x7fc00000u) : z);
+  if (!cut_k && !cut_p && !cut_typ) {
+    // ---- second pass over a row that nothing cuts: its mass and the choice ----
+    unsigned long long w = 0ull;
+    row.scan([&](int i, const float(&x)[Row<T>::VEC]) {
+#pragma unroll
+      for (int j = 0; j < Row<T>::VEC; ++j)
+        if (x[j] > -INFINITY) w += mass_of(x[j], m);
+      if (sample) {
+#pragma unroll
+        for (int q = 0; q < Row<T>::VEC; q += 4) {
+          // one Philox block holds the noise of four entries (the same numbers as gumbel_noise entry by entry)
+          const uint4 r = philox4x32(static_cast<uint32_t>(i + q) >> 2, step, static_cast<uint32_t>(seed),
+                                     static_cast<uint32_t>(seed >> 32));
+          const uint32_t bits[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (x[q + j] == -INFINITY) continue;
+            best.take(x[q + j] + tgi_sampling::gumbel_of(bits[j]), x[q + j], i + q + j);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < Row<T>::VEC; ++j)
+          if (x[j] != -INFINITY) best.take(x[j], x[j], i + j);
+      }
+    }, [&](int i, float x) {
+      if (x > -INFINITY) w += mass_of(x, m);
+      if (x != -INFINITY) best.take(sample ? x + gumbel_noise(static_cast<uint32_t>(i), step, seed) : x, x, i);
+    });
+    w = block_sum(w, red64);
+    finish(odd ? __uint_as_float(0x7fc00000u) : static_cast<float>(w) / kFixedOne);
     return;
   }
 
+  unsigned long long all = 0ull;          // mass of the row, where the second pass took it
   if (!cut_typ && !odd && m > -INFINITY && m < INFINITY) {
-    // ---- second pass: the entries within kReach of the maximum ----
+    // ---- second pass: the entries within kReach of the maximum, for top-p without top-k the mass of the row ----
     // compared as order_bits, as the keys below are: these put -0 under +0
     const uint32_t base = order_bits(m - kReach);
     auto put = [&](int i, float x) {
@@ -527,8 +514,16 @@ sample_kernel(const T* __restrict__ scores, long long row_stride, const float* _
         }
       }
     };
-    row.each(put);
-    __syncthreads();
+    if (cut_k) {
+      row.each(put);
+      __syncthreads();
+    } else {
+      row.each([&](int i, float x) {
+        all += mass_of(x, m);
+        put(i, x);
+      });
+      all = block_sum(all, red64);
+    }
     const int n = s_n;
     const int bits = 32 - __clz(order_bits(m) - base);
     auto listed = [&](auto&& f) {
@@ -547,7 +542,7 @@ sample_kernel(const T* __restrict__ scores, long long row_stride, const float* _
         if (order_bits(x) - base >= from) w += mass_of(x, m);
       });
       const unsigned long long have = block_sum(w, red64);
-      const float z_all = cut_k ? static_cast<float>(have) / kFixedOne : z;
+      const float z_all = static_cast<float>(cut_k ? have : all) / kFixedOne;
       const unsigned long long lim = static_cast<unsigned long long>(fmaxf(p * z_all, 0.f) * kFixedOne);
       // entries outside the list are left out if those above them reach the limit already
       decided = cut_k || have >= lim;
@@ -583,28 +578,18 @@ sample_kernel(const T* __restrict__ scores, long long row_stride, const float* _
     if (cut_k)
       keep_from = min(find_threshold<false, kHistCopies>(each, key, 32, m, static_cast<unsigned long long>(k), hist, tot), order_bits(m));
     if (cut_p) {
-      float zk = 0.f;
-      row.each([&](int, float x) {
-        if (order_bits(x) >= keep_from) zk += __expf(x - m);
-      });
-      zk = block_sum(zk, red);
-      const uint32_t t = find_threshold<true, kHistCopies>(each, key, 32, m,
-                                                           static_cast<unsigned long long>(fmaxf(p * zk, 0.f) * kFixedOne), hist, tot);
-      keep_from = max(keep_from, min(t, order_bits(m)));
+      bool none;
+      const float zk = static_cast<float>(kept_mass(row, m, keep_from, red64, none)) / kFixedOne;
+      const unsigned long long lim = none ? 0ull : static_cast<unsigned long long>(fmaxf(p * zk, 0.f) * kFixedOne);
+      keep_from = max(keep_from, min(find_threshold<true, kHistCopies>(each, key, 32, m, lim, hist, tot), order_bits(m)));
     }
   } else {
     if (cut_k)
       keep_from = min(row_threshold<false, T>(row, 0u, m, static_cast<unsigned long long>(k), hist, tot, list_x, list_i, &s_n, s_lo_hi),
                       order_bits(m));
     if (cut_p) {
-      float zk = z;
-      if (cut_k) {
-        zk = 0.f;
-        row.each([&](int, float x) {
-          if (order_bits(x) >= keep_from) zk += __expf(x - m);
-        });
-        zk = block_sum(zk, red);
-      }
+      bool none;
+      const float zk = static_cast<float>(cut_k || cut_typ ? kept_mass(row, m, keep_from, red64, none) : all) / kFixedOne;
       const uint32_t t = row_threshold<true, T>(row, keep_from, m, static_cast<unsigned long long>(fmaxf(p * zk, 0.f) * kFixedOne), hist,
                                                 tot, list_x, list_i, &s_n, s_lo_hi);
       keep_from = max(keep_from, min(t, order_bits(m)));
@@ -612,15 +597,20 @@ sample_kernel(const T* __restrict__ scores, long long row_stride, const float* _
   }
   uint32_t typ_bits = 0xffffffffu;
   float typ_log_z = 0.f, typ_h = 0.f;
-  if (cut_typ) typ_bits = typical_threshold<T>(row, m, keep_from, typ, red, &typ_log_z, &typ_h);
-  float zk = 0.f;
+  if (cut_typ) typ_bits = typical_threshold<T>(row, m, keep_from, typ, red64, &typ_log_z, &typ_h);
+  unsigned long long w = 0ull;
+  bool none = false;
   row.each([&](int i, float x) {
     if (order_bits(x) < keep_from || x == -INFINITY) return;
     if (cut_typ && __float_as_uint(fabsf(-(x - m - typ_log_z) - typ_h)) > typ_bits) return;
-    zk += __expf(x - m);
+    const float e = __expf(x - m);
+    if (e == e) w += static_cast<unsigned long long>(e * kFixedOne);
+    else none = true;
     best.take(sample ? x + gumbel_noise(static_cast<uint32_t>(i), step, seed) : x, x, i);
   });
-  finish(block_sum(zk, red));
+  none = __syncthreads_or(none);
+  w = block_sum(w, red64);
+  finish(none ? __uint_as_float(0x7fc00000u) : static_cast<float>(w) / kFixedOne);
 }
 
 size_t sample_bytes(int V, bool rep) {
@@ -655,19 +645,21 @@ extern "C" {
 
 // Fused repetition penalty / temperature / top-k / top-p / sampling; any of temperature, top_k, top_p, do_sample, seeds, steps
 // may be null (stage off).  `rep` [B] (null: none) with `history` int64 [B, L].  `is_fp32` selects the element type of
-// `scores`.  Up to 148 rows (one per SM) run on 1024 threads each, more on 512, two or more rows to an SM.
+// `scores`.  As many rows as the device has SMs run on 1024 threads each, more on 512, two rows to an SM; results are the same.
 int tgi_sample(const void* scores, long long row_stride, int is_fp32, const float* temperature, const int* top_k,
                const float* top_p, const float* typical_p, const unsigned char* do_sample, const long long* seeds,
                const int* steps, const long long* history, int L, const float* rep, long long* ids, float* logprob, int B, int V,
                cudaStream_t stream) {
   if (B <= 0) return 0;
   if (V <= 0) return -10;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -2;
   if (is_fp32)
-    return B <= 148 ? launch_sample<float, 1024>(scores, row_stride, temperature, top_k, top_p, typical_p, do_sample, seeds, steps,
+    return B <= sms ? launch_sample<float, 1024>(scores, row_stride, temperature, top_k, top_p, typical_p, do_sample, seeds, steps,
                                                  history, L, rep, ids, logprob, B, V, stream)
                     : launch_sample<float, 512>(scores, row_stride, temperature, top_k, top_p, typical_p, do_sample, seeds, steps,
                                                 history, L, rep, ids, logprob, B, V, stream);
-  return B <= 148 ? launch_sample<__nv_bfloat16, 1024>(scores, row_stride, temperature, top_k, top_p, typical_p, do_sample, seeds,
+  return B <= sms ? launch_sample<__nv_bfloat16, 1024>(scores, row_stride, temperature, top_k, top_p, typical_p, do_sample, seeds,
                                                        steps, history, L, rep, ids, logprob, B, V, stream)
                   : launch_sample<__nv_bfloat16, 512>(scores, row_stride, temperature, top_k, top_p, typical_p, do_sample, seeds,
                                                       steps, history, L, rep, ids, logprob, B, V, stream);
