@@ -1,5 +1,5 @@
 """Sampler kernel: what a row gives depends on nothing but the row: not on the signs of zeros among the listed entries, on the other
-rows, on where it lies in memory, nor on the order in which penalised ids are met."""
+rows, on where it lies in memory, nor on the order in which penalised ids are met; histories on both sides of the list's size."""
 import pytest
 import torch
 
@@ -75,3 +75,21 @@ def test_order_of_the_history(rows, cut):
     for _ in range(4):
         history = history[:, torch.randperm(1500, device="cuda", generator=g)]
         _same(K.fused_sample(x, history=history, repetition_penalty=pen, **kw), first)
+
+
+@pytest.mark.parametrize("rows", [3, 150])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("ids", [2048, 2049, 3072, 3073, 6000])
+@pytest.mark.parametrize("cut", ["none", "top_p", "both", "typical"])
+def test_long_histories(rows, dtype, ids, cut):
+    """Against a penalised copy of the scores."""
+    from tgi_b200.ops import cuda as K
+
+    K.load()
+    V = 32003
+    g = torch.Generator(device="cuda").manual_seed(ids)
+    x = (torch.randn(rows, V, device="cuda", generator=g) * 2).to(dtype)
+    history = torch.rand(rows, V, device="cuda", generator=g).argsort(1)[:, :ids]
+    pen = torch.tensor([1.3, 0.8, 1.0], device="cuda").repeat(rows)[:rows]
+    kw = _params(rows, cut)
+    _same(K.fused_sample(x, history=history, repetition_penalty=pen, **kw), K.fused_sample(K.penalties(x, history, pen, None), **kw))

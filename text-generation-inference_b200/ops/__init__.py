@@ -342,7 +342,7 @@ def fused_sample(scores, temperature=None, top_k=None, top_p=None, do_sample=Non
 
 def fused_sample_penalises(scores) -> bool:
     """Whether ``fused_sample`` takes the repetition penalty for these scores (otherwise ``penalties`` comes first)."""
-    return scores.dtype in (torch.float32, torch.bfloat16) and scores.shape[1] <= native().SAMPLE_PENALTY_MAX_VOCAB
+    return scores.dtype in (torch.float32, torch.bfloat16)
 
 
 def penalties(scores, history, repetition_penalty=None, frequency_penalty=None):

@@ -36,24 +36,18 @@ using tgi_sampling::philox4x32;
 
 // A row of logits as the sampler sees it.  Penalised entries are met once each, apart from the others: a 16-byte load that
 // holds some (the ids of a 1000-token history are in most warps' loads) leaves them out, and their scores, computed with
-// one division each when the row is set up, follow from a list.  A history with more ids than the list holds takes
-// the division where an entry is read.
+// one division each when the row is set up, follow from a list.
 template <typename T>
 struct Row {
   const T* p;
   int V;
   float inv_t;
-  float rp;                    // repetition penalty of the ids whose bit is set in `marks` (null: none)
-  const uint32_t* marks;
-  const float* pen_x;          // scores of the penalised entries and their indices, n_pen of them (-1: not listed)
+  const uint32_t* marks;       // a bit per id: penalised (null: none)
+  const float* pen_x;          // scores of the penalised entries and their indices, n_pen of them in any order
   const int* pen_i;
   int n_pen;
   static constexpr int VEC = 16 / sizeof(T);
 
-  __device__ __forceinline__ float penalised(int i) const {
-    const float x = static_cast<float>(p[i]);
-    return (x < 0.f ? x * rp : x / rp) * inv_t;
-  }
   __device__ __forceinline__ int vectors() const { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 ? V / VEC : 0; }
   __device__ __forceinline__ void unpack(const uint4& raw, int v, float (&x)[VEC]) const {
     const T* e = reinterpret_cast<const T*>(&raw);
@@ -62,20 +56,9 @@ struct Row {
     if (marks == nullptr) return;
     const uint32_t bits = marks[(v * VEC) >> 5] >> ((v * VEC) & 31);
     if ((bits & ((1u << VEC) - 1u)) == 0u) return;
-    if (n_pen >= 0) {
 #pragma unroll
-      for (int j = 0; j < VEC; ++j)
-        if ((bits >> j) & 1u) x[j] = -INFINITY;
-    } else {
-#pragma unroll 1
-      for (int j = 0; j < VEC; ++j) {
-        if (!((bits >> j) & 1u)) continue;
-        const float y = penalised(v * VEC + j);
-#pragma unroll
-        for (int q = 0; q < VEC; ++q)
-          if (q == j) x[q] = y;
-      }
-    }
+    for (int j = 0; j < VEC; ++j)
+      if ((bits >> j) & 1u) x[j] = -INFINITY;
   }
   // fv(first index, scores) for runs of VEC entries (16-byte loads, four in flight per thread), f1(index, score) for
   // the others; -inf may stand in for an entry that is met elsewhere
@@ -97,10 +80,8 @@ struct Row {
         }
       }
     }
-    for (int i = nvec * VEC + threadIdx.x; i < V; i += step) {
+    for (int i = nvec * VEC + threadIdx.x; i < V; i += step)
       if (marks == nullptr || ((marks[i >> 5] >> (i & 31)) & 1u) == 0u) f1(i, static_cast<float>(p[i]) * inv_t);
-      else if (n_pen < 0) f1(i, penalised(i));
-    }
     for (int j = threadIdx.x; j < n_pen; j += step) f1(pen_i[j], pen_x[j]);
   }
   template <typename F>
@@ -127,7 +108,10 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long v, un
 constexpr int kHistCopies = 16;          // of a 256-bin histogram: one per warp or pair of warps
 constexpr int kBins = 1024, kBinCopies = 4;      // the same memory as bins of 1/32 below the maximum
 constexpr float kBinScale = 32.f;
-constexpr int kPenalised = 2048;         // ids of a history that are listed
+// History that is listed: with it and 160k bits of marks a row takes 108 KB, two rows to an SM.  The caller turns to a penalised
+// copy of the scores for longer ones; dividing where an entry is read instead took 3247 us for typical-p over 256 rows x 128256 with
+// 4096 ids and 454 for top-k, the copy and the sampler 1170 and 201.
+constexpr int kPenalised = 3072;
 constexpr float kFixedOne = 1099511627776.f;   // 2^40
 constexpr float kReach = 8.f;            // entries below the maximum by more than this are not listed
 constexpr int kList = 4096;              // listed entries
@@ -397,9 +381,9 @@ sample_kernel(const T* __restrict__ scores, long long row_stride, const float* _
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int kWarps = THREADS / 32;
   const float temp = temperature != nullptr ? temperature[b] : 1.f;
-  Row<T> row{scores + static_cast<size_t>(b) * row_stride, V, 1.f / (temp > 0.f ? temp : 1.f), 1.f, nullptr, pen_x, pen_i, 0};
+  Row<T> row{scores + static_cast<size_t>(b) * row_stride, V, 1.f / (temp > 0.f ? temp : 1.f), nullptr, pen_x, pen_i, 0};
   if (rep != nullptr && rep[b] != 1.f) {
-    row.rp = rep[b];
+    const float rp = rep[b];
     row.marks = marks;
     for (int w = threadIdx.x; w < (V + 31) / 32; w += THREADS) marks[w] = 0u;
     if (threadIdx.x == 0) s_n = 0;
@@ -410,14 +394,13 @@ sample_kernel(const T* __restrict__ scores, long long row_stride, const float* _
       if (t < 0 || t >= V) continue;
       const uint32_t bit = 1u << (t & 31);
       if (atomicOr(&marks[t >> 5], bit) & bit) continue;         // met before
-      const int at = atomicAdd(&s_n, 1);
-      if (at < kPenalised) {
-        pen_x[at] = row.penalised(static_cast<int>(t));
-        pen_i[at] = static_cast<int>(t);
-      }
+      const int at = atomicAdd(&s_n, 1);                         // below L <= kPenalised
+      const float x = static_cast<float>(row.p[t]);
+      pen_x[at] = (x < 0.f ? x * rp : x / rp) * row.inv_t;
+      pen_i[at] = static_cast<int>(t);
     }
     __syncthreads();
-    row.n_pen = s_n <= kPenalised ? s_n : -1;
+    row.n_pen = s_n;
     __syncthreads();
   }
   const int k = top_k != nullptr ? top_k[b] : 0;
@@ -625,7 +608,7 @@ int launch_sample(const void* scores, long long row_stride, const float* tempera
                   cudaStream_t stream) {
   auto kern = sample_kernel<T, THREADS>;
   const size_t smem = sample_bytes(V, rep != nullptr);
-  if (smem > 200 * 1024) return -10;
+  if (smem > 200 * 1024 || (rep != nullptr && L > kPenalised)) return -10;
   static std::atomic<unsigned long long> attr_set{0};      // per device: the opt-in to the largest size that is launched
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return -2;
@@ -644,7 +627,7 @@ int launch_sample(const void* scores, long long row_stride, const float* tempera
 extern "C" {
 
 // Fused repetition penalty / temperature / top-k / top-p / sampling; any of temperature, top_k, top_p, do_sample, seeds, steps
-// may be null (stage off).  `rep` [B] (null: none) with `history` int64 [B, L].  `is_fp32` selects the element type of
+// may be null (stage off).  `rep` [B] (null: none) with `history` int64 [B, L], L <= 3072.  `is_fp32` selects the element type of
 // `scores`.  As many rows as the device has SMs run on 1024 threads each, more on 512, two rows to an SM; results are the same.
 int tgi_sample(const void* scores, long long row_stride, int is_fp32, const float* temperature, const int* top_k,
                const float* top_p, const float* typical_p, const unsigned char* do_sample, const long long* seeds,

@@ -851,8 +851,9 @@ def argmax_logprob(logits):
     return ids, lp
 
 
-# vocabularies up to this size: the sampler marks the penalised ids of a row in a bitmap in shared memory
+# vocabularies and histories up to these sizes: the sampler marks and lists the penalised ids of a row in shared memory
 SAMPLE_PENALTY_MAX_VOCAB = 1 << 19
+SAMPLE_PENALTY_MAX_HISTORY = 3072
 
 
 def fused_sample(scores: torch.Tensor, temperature=None, top_k=None, top_p=None, do_sample=None, seeds=None, steps=None,
@@ -860,7 +861,8 @@ def fused_sample(scores: torch.Tensor, temperature=None, top_k=None, top_p=None,
     """Temperature, top-k, top-p and sampling (Gumbel-max with a counter-based generator keyed by the
     request's seed and step) in one kernel; returns ``(ids int64 [B], logprobs fp32 [B])``.  Any stage
     whose tensor is ``None`` is off; rows with ``do_sample == 0`` take the argmax of the filtered scores.
-    ``repetition_penalty`` (fp32 ``[B]``) is applied first, to the ids in ``history[B, L]``, as ``penalties`` does."""
+    ``repetition_penalty`` (fp32 ``[B]``) is applied first, to the ids in ``history[B, L]``, as ``penalties`` does (and by it, on a
+    copy of the scores, for sizes that the kernel has no room for)."""
     lib = load()
     assert scores.dim() == 2 and scores.stride(1) == 1 and scores.dtype in (torch.float32, torch.bfloat16)
     B, V = scores.shape
@@ -879,6 +881,9 @@ def fused_sample(scores: torch.Tensor, temperature=None, top_k=None, top_p=None,
     do_sample, seeds = as_(do_sample, torch.uint8), as_(seeds, torch.int64)
     repetition_penalty = as_(repetition_penalty, torch.float32)
     history = None if repetition_penalty is None else as_(history, torch.int64)
+    if history is not None and (V > SAMPLE_PENALTY_MAX_VOCAB or history.shape[1] > SAMPLE_PENALTY_MAX_HISTORY):
+        scores = penalties(scores, history, repetition_penalty, None)
+        history = repetition_penalty = None
     _check(lib.tgi_sample(_ptr(scores), c_ll(scores.stride(0)), c_int(1 if scores.dtype == torch.float32 else 0),
                           _ptr(temperature), _ptr(top_k), _ptr(top_p), _ptr(typical_p), _ptr(do_sample), _ptr(seeds),
                           _ptr(steps), _ptr(history), c_int(0 if history is None else history.shape[1]), _ptr(repetition_penalty),
