@@ -690,8 +690,9 @@ int skinny_int4(const void* X, const void* W, const void* scale, const void* zp,
                        M - m0 < kInt4Tokens ? M - m0 : kInt4Tokens, N, K, settled && m0 == 0, status);
     a.has_zp = zp != nullptr;
     a.group_units = group / 128;
-    const int rc = launch<kInt4>(Operands{static_cast<const __nv_bfloat16*>(X) + static_cast<size_t>(m0) * K, 2LL * K, W, nullptr, 0,
-                                          scale, zp}, a, max_ctas, stream);
+    const Operands o{static_cast<const __nv_bfloat16*>(X) + static_cast<size_t>(m0) * K, 2LL * K, W, nullptr, 0, scale, zp};
+    // all tokens of a call in the same chains of MMAs: equal tokens give equal rows
+    const int rc = M > kInt4Tokens ? launch_nt<kInt4, 2>(o, a, max_ctas, stream) : launch<kInt4>(o, a, max_ctas, stream);
     if (rc) return rc;
   }
   return 0;
