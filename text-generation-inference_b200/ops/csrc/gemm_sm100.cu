@@ -841,14 +841,21 @@ int launch(const void* X, const float* xs_t, int xs_pitch, const void* W, const 
   if (grid < 1) grid = 1;
   int whole_tiles = 0;
   if (tiles > max_workers && !(FP8 && M > Cfg::TM)) {
-    // Whole tiles in rounds, or equal shares whose cut tiles are put together through global memory.  On B200 the latter costs
-    // about 34 us whatever the sizes, a K block about 0.5 us.  Equal shares / whole tiles in us: 28672 x 4096 bf16 (112 pair tiles on
-    // 74 pairs) with 201 tokens 76 / 56, 128256 x 4096 with 201 237 / 215 and with 64 195 / 164, 57344 x 8192 fp8 with 64 104 / 84,
-    // with 256 143 / 136.  Prompts in fp8 (several token tiles) keep equal shares: there the two are equally fast (3300 tokens of
-    // a 70B model 34 / 34 ms), and a model that quantises its activations anew for every product would change its results.
+    // Whole tiles in rounds, or equal shares whose cut tiles are put together through global memory, which costs 10 to 20 us.  How many
+    // K blocks of 128 bytes that is depends on what a worker needs for one: 0.2 us in bf16, 0.4 in block-scaled fp8 on pairs, 0.6 in fp8
+    // with promotion.  Measured on B200, captured, equal shares / whole tiles in us at the blocks that the latter take on top:
+    //   bf16 pairs, 201 tokens         28672 x 4096  (31) 66 / 56     19200 x 4096 (63) 52 / 49      57344 x 8192 (124) 242 / 264
+    //   bf16, 64 tokens                128256 x 4096 (39) 182 / 170   57344 x 8192 (62) 163 / 153    38400 x 8192 (126) 114 / 115
+    //   fp8 block-scaled, 201 tokens   28672 x 4096  (15) 54 / 41     28672 x 8192 (31) 78 / 70      57344 x 8192 (62) 150 / 162
+    //   fp8 block-scaled, 64 tokens    57344 x 8192  (31) 91 / 87     38400 x 8192 (63) 68 / 66
+    //   fp8 promotion, 201 tokens      28672 x 4096  (15) 61 / 52     24576 x 4096 (22) 58 / 52      38400 x 4096 (31) 70 / 75
+    //   fp8 promotion, 64 tokens       38400 x 1024  (7) 28 / 25      152064 x 3584 (27) 120 / 130   38400 x 4096 (31) 44 / 54
+    // Prompts in fp8 (several token tiles) keep equal shares, so that their results stay what they were: a model that quantises its
+    // activations anew for every product carries a last bit far.  Whole tiles would save them 6 to 27 us at up to 31 blocks on top.
+    constexpr int kWorth = !FP8 ? 68 : !MX ? 24 : PAIR ? 40 : 68;
     const int rounds = (tiles + max_workers - 1) / max_workers;
     const long long extra = static_cast<long long>(rounds) * KBn - (units + max_workers - 1) / max_workers;
-    if (extra * 0.5 < 34.0) {
+    if (extra < kWorth) {
       whole_tiles = 1;
       grid = (tiles + rounds - 1) / rounds;
     }
