@@ -157,3 +157,96 @@ def test_equal_tokens_give_equal_rows(fmt):
         else:
             y = K.gemm_fp8_block(*K.fp8_quant_act(x), w.to(torch.float8_e4m3fn), torch.ones(5, 16, device=dev()))
         assert torch.equal(y, y[:1].expand(M, -1)), M
+
+
+@pytest.mark.parametrize("fmt", ["bf16", "fp8"])
+@pytest.mark.parametrize("M,N,Kd", [(200, 8192, 8192), (300, 4096, 8192)])
+def test_settled_weights_on_pairs(fmt, M, N, Kd):
+    """At least 32 tiles of 256 x 256 run on CTA pairs: both CTAs' weights go to the leader's barriers ahead of the wait, with many more K
+    blocks to a pair than stages."""
+    from tgi_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(M)
+    norm = torch.ones(Kd, device=dev(), dtype=torch.bfloat16)
+    xs = [torch.randn(M, Kd, device=dev(), generator=g).to(torch.bfloat16) for _ in range(3)]
+    w = torch.randn(N, Kd, device=dev(), generator=g) * 0.02
+    w = ((w * 2000).clamp(-440, 440).to(torch.float8_e4m3fn), torch.full((N // 128, Kd // 128), 2.0 ** -11, device=dev())) \
+        if fmt == "fp8" else w.to(torch.bfloat16)
+
+    def step(settled):
+        if fmt == "fp8":
+            return [K.gemm_fp8_block(*K.rms_norm_quant(x, None, norm, 1e-5)[:2], *w, settled=settled) for x in xs]
+        return [K.gemm_bf16(K.rms_norm(x, None, norm, 1e-5)[0], w, settled=settled) for x in xs]
+
+    want = step(False)
+    assert K.load().tgi_gemm_last_grid() % 2 == 0
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = step(True)
+    for _ in range(10):
+        for y in got:
+            y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert K.check_status(dev()) == 0 and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("batch", [3, 40, 200])
+@pytest.mark.parametrize("pages", [torch.bfloat16, torch.float8_e4m3fn])
+def test_settled_weights_behind_decode_attention(batch, pages):
+    """A captured chain of decode attention (split and merged for few sequences) and products that fetch their weights meanwhile."""
+    from tgi_b200.ops import cuda as K
+
+    heads, kv_heads, L = 16, 4, 1500 if batch < 100 else 200
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    blocks = (L + 15) // 16
+    kc, vc = (torch.randn(batch * blocks, 16, kv_heads, 128, device=dev(), generator=g).to(pages) for _ in range(2))
+    table = torch.randperm(batch * blocks, device=dev(), generator=g).int().view(batch, blocks)
+    kv = (torch.rand(batch, device=dev(), generator=g) * (L - 1) + 1).int()
+    cu = torch.arange(batch + 1, device=dev(), dtype=torch.int32)
+    one = torch.ones(kv_heads, device=dev()) if pages != torch.bfloat16 else None
+    ws = [(torch.randn(heads * 128, heads * 128, device=dev(), generator=g) * 0.05).to(torch.bfloat16) for _ in range(4)]
+    x = torch.randn(batch, heads * 128, device=dev(), generator=g).to(torch.bfloat16)
+
+    def step(settled):
+        y = x
+        for w in ws:
+            o = K.paged_attention(y.view(batch, heads, 128), kc, vc, table, cu, kv, 128 ** -0.5, -1, 0.0, one, one, 1, L)
+            y = K.gemm_bf16(o.view(batch, -1), w, settled=settled)
+        return y
+
+    want = step(False)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = step(True)
+    for _ in range(20):
+        got.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert K.check_status(dev()) == 0 and torch.equal(got, want)
+
+
+def test_fp8_tokens_alone_and_among_others():
+    """From 9 tokens on a token's product is the same in every batch up to 128, to the bit; with up to 8 its sums have another order, so
+    it is the same but for roundings."""
+    from tgi_b200.ops import cuda as K
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    N, Kd = 1024, 4096
+    q, s = K.fp8_quant_act(torch.randn(128, Kd, device=dev(), generator=g).to(torch.bfloat16))
+    wq = (torch.randn(N, Kd, device=dev(), generator=g) * 60).clamp(-440, 440).to(torch.float8_e4m3fn)
+    ws = torch.exp2(torch.randint(-12, -6, (N // 128, Kd // 128), device=dev(), generator=g).float())
+
+    def first(M):
+        scales = K.alloc_act_scales(M, Kd // 128, dev())
+        scales.copy_(s[:M])
+        return K.gemm_fp8_block(q[:M].contiguous(), scales, wq, ws)
+
+    most = first(128)
+    for M in (9, 16, 17, 64):
+        assert torch.equal(first(M), most[:M]), M
+    x = (q.double().view(128, -1, 128) * s.double()[:, :, None]).view(128, Kd)[:8]
+    w = (wq.double().view(N, -1, 128) * ws.double().repeat_interleave(128, 0)[:N, :, None]).view(N, Kd)
+    for M in (1, 5, 8):
+        bound = (x[:M] @ w.t()).abs() * 2 ** -7 + (x[:M].abs() @ w.abs().t()) * 2 ** -15
+        assert ((first(M).double() - most[:M].double()).abs() <= bound).all(), M
