@@ -240,6 +240,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         const int blk0 = walk.first(p), nb = walk.count(p);
         for (int c = 0; c < chunks && ok; ++c) {
           for (int t = 0; t < nb; ++t, ++issued, r.next()) {
+            // the ring is full of settled weights: room comes when the launch ahead has ended, however long that takes
+            if (a.settled && issued == STAGES) tgi::pdl_wait();
             ok = mbar_wait(&empty[r.slot], r.phase);
             if (!ok) {
               report(a.status, kErrProducerWait);
