@@ -1,5 +1,5 @@
 """Sampler kernel: what a row gives depends on nothing but the row: not on the signs of zeros among the listed entries, on the other
-rows, on where it lies in memory, nor on the order in which penalised ids are met; histories on both sides of the list's size."""
+rows, on where it lies in memory, nor on the order in which penalised ids are met; histories on both sides of the list's size, NaN."""
 import pytest
 import torch
 
@@ -93,3 +93,25 @@ def test_long_histories(rows, dtype, ids, cut):
     pen = torch.tensor([1.3, 0.8, 1.0], device="cuda").repeat(rows)[:rows]
     kw = _params(rows, cut)
     _same(K.fused_sample(x, history=history, repetition_penalty=pen, **kw), K.fused_sample(K.penalties(x, history, pen, None), **kw))
+
+
+@pytest.mark.parametrize("vocab", [5, 1000, 4099])
+@pytest.mark.parametrize("cut", CUTS)
+def test_nan_among_penalised_entries(vocab, cut):
+    """NaN has one place in the order (under every number that is not negative), whichever way an entry is met."""
+    from tgi_b200.ops import cuda as K
+
+    K.load()
+    g = torch.Generator(device="cuda").manual_seed(vocab)
+    x = torch.randn(12, vocab, device="cuda", generator=g) * 3
+    x[:, torch.randperm(vocab, device="cuda", generator=g)[:2]] = float("nan")
+    x[3] = float("nan")
+    x[4, 0] = float("inf")
+    kw = _params(12, cut)
+    if "top_k" in kw:
+        kw["top_k"] = torch.tensor([1, 2, 3, 4], device="cuda", dtype=torch.int32).repeat(3)
+    history = torch.randint(0, vocab, (12, 40), device="cuda", generator=g)
+    history[:, :2] = x[0].isnan().nonzero()[:2, 0]
+    pen = torch.tensor([1.2, 0.7, 1.0], device="cuda").repeat(4)
+    got, want = (K.fused_sample(x, history=history, repetition_penalty=pen, **kw), K.fused_sample(K.penalties(x, history, pen, None), **kw))
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1].nan_to_num(7e7), want[1].nan_to_num(7e7))

@@ -282,13 +282,17 @@ __device__ uint32_t row_threshold(const Row<T>& row, uint32_t floor_bits, float 
                                            m, lim, hist, tot);
 }
 
+// The image for rows that may hold NaN: below every number that is not negative.  The bits of a NaN depend on the instructions that the
+// compiler makes of a product or a division, so order_bits would differ from pass to pass.
+__device__ __forceinline__ uint32_t key_bits(float x) { return x == x ? order_bits(x) : 0x7fffffffu; }
+
 // Mass of the entries of a row from `keep_from` on; `none`: some of them has no mass (NaN, or an infinite maximum).
 template <typename T>
 __device__ unsigned long long kept_mass(const Row<T>& row, float m, uint32_t keep_from, unsigned long long* red, bool& none) {
   unsigned long long w = 0ull;
   bool odd = false;
   row.each([&](int, float x) {
-    if (order_bits(x) < keep_from) return;
+    if (key_bits(x) < keep_from) return;
     const float e = __expf(x - m);
     if (e == e) w += static_cast<unsigned long long>(e * kFixedOne);
     else odd = true;
@@ -308,7 +312,7 @@ __device__ uint32_t typical_threshold(const Row<T>& row, float m, uint32_t keep_
   unsigned long long w = 0ull, s = 0ull;
   bool odd = false;
   row.each([&](int, float x) {
-    if (order_bits(x) < keep_from || x == -INFINITY) return;
+    if (key_bits(x) < keep_from || x == -INFINITY) return;
     const float e = __expf(x - m);
     if (e == e) {
       w += static_cast<unsigned long long>(e * kFixedOne);
@@ -331,7 +335,7 @@ __device__ uint32_t typical_threshold(const Row<T>& row, float m, uint32_t keep_
     const uint32_t mid = lo + ((hi - lo) >> 1);
     unsigned long long acc = 0ull;
     row.each([&](int, float x) {
-      if (order_bits(x) >= keep_from && x != -INFINITY) {
+      if (key_bits(x) >= keep_from && x != -INFINITY) {
         const float lp = x - m - log_z;
         if (__float_as_uint(fabsf(-lp - H)) <= mid) acc += mass_of(x, m);
       }
@@ -555,7 +559,7 @@ sample_kernel(const T* __restrict__ scores, long long row_stride, const float* _
     // distances from the maximum say nothing: radix select over the row
     auto each = [&](auto&& f) { row.each(f); };
     auto key = [&](float x, uint32_t& out) {
-      out = order_bits(x);
+      out = key_bits(x);
       return out >= keep_from;
     };
     if (cut_k)
@@ -584,7 +588,7 @@ sample_kernel(const T* __restrict__ scores, long long row_stride, const float* _
   unsigned long long w = 0ull;
   bool none = false;
   row.each([&](int i, float x) {
-    if (order_bits(x) < keep_from || x == -INFINITY) return;
+    if (key_bits(x) < keep_from || x == -INFINITY) return;
     if (cut_typ && __float_as_uint(fabsf(-(x - m - typ_log_z) - typ_h)) > typ_bits) return;
     const float e = __expf(x - m);
     if (e == e) w += static_cast<unsigned long long>(e * kFixedOne);
