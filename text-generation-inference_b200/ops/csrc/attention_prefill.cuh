@@ -75,10 +75,11 @@ __device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&r)[32]) {
   tmem_ld_wait(r);
 }
 
-// 2^x on the FMA pipe, for x <= 0: the special-function unit does 16 ex2 per cycle and SM and is the busiest
-// unit of a tile (16 K exponentials), so every POLY-th probability is computed this way instead.  Round x to
-// the nearest integer with the 1.5 * 2^23 trick, evaluate a cubic for 2^f on [-0.5, 0.5] (relative error 1.4e-4,
-// well under the 16-bit rounding of P) and add the integer to the exponent field.
+// 2^x on the FMA pipe, for x <= 8 (the bf16 kernel's rows may outgrow their reference by 2^8, the e4m3 kernel's x are <= 0): the
+// special-function unit does 16 ex2 per cycle and SM and is the busiest unit of a tile (16 K exponentials), so every POLY-th
+// probability is computed this way instead, as in FlashAttention-4.  Round x to the nearest integer with the 1.5 * 2^23 trick,
+// evaluate a cubic for 2^f on [-0.5, 0.5] (relative error 1.4e-4, well under the 16-bit rounding of P) and add the integer to the
+// exponent field (the reduction of W. J. Cody and W. Waite, Software Manual for the Elementary Functions, 1980).
 __device__ __forceinline__ float poly_exp2(float x) {
   x = fmaxf(x, -125.f);
   const float t = x + 12582912.f;

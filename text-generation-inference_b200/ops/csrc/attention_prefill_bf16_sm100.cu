@@ -14,7 +14,8 @@
 //   O += P V       tcgen05.mma, M 128 x N 128 (head dim) x K 128 (keys), accumulated in TMEM over the chain; V is taken as the
 //                  MN-major operand, i.e. exactly as the page boxes land in shared memory (rows = tokens, 128 bytes = 64
 //                  head elements).  A chain's reference maximum moves only when a row's maximum has outgrown it by 2^8 (P is
-//                  then up to 256: the relative precision of its 16 bits is the same); its warps then rescale O in TMEM
+//                  then up to 256: the relative precision of its 16 bits is the same); its warps then rescale O in TMEM (rescaling only when the
+//                  maximum has grown by a threshold: FlashAttention-4)
 //   out            (O_even a_even + O_odd a_odd) / l with a = 2^(m_chain - m)
 // What bounds it is the softmax's instructions (about six per score, 16 K scores a tile, against 512 cycles of MMA).  While a chain
 // waits for its scores or for room for P the other one computes.  A single chain whose eight warps shared a tile, with the running
@@ -131,7 +132,6 @@ prefill_chains_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_cons
     tmem_relinquish();
   }
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

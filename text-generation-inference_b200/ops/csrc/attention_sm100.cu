@@ -332,7 +332,6 @@ template <int D, bool FP8>
 __global__ void __launch_bounds__(128)
 prefill_kernel(Params p) {
   tgi::pdl_wait();      // inputs come from earlier kernels of the stream
-  tgi::pdl_trigger();   // let the next kernel be placed while this one runs
   extern __shared__ __align__(128) uint8_t smem[];
   using S = Smem<D, FP8>;
   uint16_t* sQ = reinterpret_cast<uint16_t*>(smem);

@@ -84,7 +84,6 @@ row_norm_store_kernel(const T* __restrict__ proj, const int* __restrict__ positi
                       const float* __restrict__ wq, const float* __restrict__ wk, T* __restrict__ q_out,
                       T* __restrict__ k_cache, T* __restrict__ v_cache, RowNorm p) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   __shared__ float red[66];
   const int t = blockIdx.x;
   const T* row = proj + static_cast<size_t>(t) * p.ld;
@@ -162,7 +161,6 @@ __global__ void __launch_bounds__(256)
 output_gate_kernel(const T* __restrict__ x, const T* __restrict__ gate, long long ld, T* __restrict__ out, long long n, int H,
                    int pitch, int width) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   constexpr int N = VEC ? Vec<T>::N : 1;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   const unsigned cols = static_cast<unsigned>(H * width);
@@ -226,7 +224,6 @@ latent_store_kernel(const T* __restrict__ proj, const float* __restrict__ weight
                     const T* __restrict__ q_in, T* __restrict__ q_out, T* __restrict__ q_full,
                     const float* __restrict__ cq_weight, T* __restrict__ cq_out, Latent p) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int t = blockIdx.x, lane = threadIdx.x & 31, warps = (blockDim.x >> 5) * gridDim.y;
   const int warp = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const T* row = proj + static_cast<size_t>(t) * p.ld;
@@ -353,7 +350,6 @@ __global__ void __launch_bounds__(256)
 map_store_kernel(const T* __restrict__ proj, const int* __restrict__ slots, T* __restrict__ q_out, T* __restrict__ k_cache,
                  T* __restrict__ v_cache, Maps p) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   constexpr int N = VEC ? Vec<T>::N : 1;
   const int t = blockIdx.x;
   const T* row = proj + static_cast<size_t>(t) * p.ld;
@@ -387,7 +383,6 @@ __global__ void __launch_bounds__(256)
 map_difference_kernel(const T* __restrict__ a, const T* __restrict__ gate, long long ld_gate, T* __restrict__ out, long long jobs,
                       int H, int pitch, int vdim, float lambda, float factor, float eps) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int l = threadIdx.x % L;
   const long long job = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / L;
   const bool on = job < jobs;                              // lanes past the last head stay for the exchanges

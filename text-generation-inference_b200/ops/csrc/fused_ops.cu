@@ -296,7 +296,6 @@ rope_cache_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__
                   const float* __restrict__ v_scale, int Hq, int Hkv, int D, int rot, int neox, long long num_slots,
                   int max_pos) {
   tgi::pdl_wait();      // inputs come from earlier kernels of the stream
-  tgi::pdl_trigger();   // let the next kernel be placed while this one runs
   const int t = blockIdx.x;
   // a position beyond the rotary table (operator asked for more tokens than the model supports) reads
   // the table's last row instead of running off its end
@@ -370,7 +369,6 @@ rope_cache_vec_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restri
                       const float* __restrict__ k_scale, const float* __restrict__ v_scale, int Hq, int Hkv, int D,
                       long long num_slots, int max_pos) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int t = blockIdx.x;
   const int pos = min(max(positions[t], 0), max_pos - 1);
   const long long slot = slots[t];
@@ -437,7 +435,6 @@ __global__ void __launch_bounds__(256)
 embedding_kernel(const int* __restrict__ ids, const __nv_bfloat16* __restrict__ table, __nv_bfloat16* __restrict__ out,
                  int H, int rows) {
   tgi::pdl_wait();      // inputs come from earlier kernels of the stream
-  tgi::pdl_trigger();   // let the next kernel be placed while this one runs
   const int t = blockIdx.x;
   int id = ids[t];
   if (id < 0 || id >= rows) id = rows - 1;  // self-check: clamp instead of reading out of bounds
@@ -452,7 +449,6 @@ __global__ void __launch_bounds__(1024)
 argmax_logprob_kernel(const T* __restrict__ logits, long long* __restrict__ ids, float* __restrict__ logprob, int V,
                       long long row_stride) {
   tgi::pdl_wait();      // inputs come from earlier kernels of the stream
-  tgi::pdl_trigger();   // let the next kernel be placed while this one runs
   __shared__ float s_m[32], s_s[32];
   __shared__ int s_i[32];
   const T* row = logits + static_cast<size_t>(blockIdx.x) * row_stride;
@@ -571,7 +567,6 @@ __global__ void __launch_bounds__(256) qk_norm_kernel(__nv_bfloat16* qkv, long l
                                                       const __nv_bfloat16* qw, const __nv_bfloat16* kw, int q_head_stride,
                                                       int k_head_stride, float eps, float w_offset, int layer) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int lane = threadIdx.x & 31;
   const long long unit = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int heads = nh + nkv;

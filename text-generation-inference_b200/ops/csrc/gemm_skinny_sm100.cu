@@ -28,8 +28,8 @@
 // is multiplied by the fp32 scale.
 //
 // Settled weights (gemm_skinny.h) are fetched from the moment the launch ahead lets this one be placed: up to 28 MB are in
-// shared memory when its tokens are there.  A step of an 8B model for one sequence 1887 -> 1753 us, for 19 2255 -> 2214, 70B fp8 for
-// eight 1873 -> 1815, 8B 4-bit for twelve 1836 -> 1788.
+// shared memory when its tokens are there.  Steps without it / with it, us: 8B for one sequence 1917 / 1762, for 19 2230 / 2175, 70B fp8
+// for eight 1877 / 1827, 8B 4-bit for twelve 1835 / 1790.
 //
 // Waits are bounded (sm100.cuh): on expiry the status word is set and the launch ends with wrong results, never late.
 #include <cuda_fp16.h>
@@ -63,13 +63,14 @@ struct Cfg {
   static constexpr int kScaleBytes = FMT == kInt4 ? 16 * kRows * 2 : 0;               // of a stage, zero points as many
   static constexpr int kStageBytes = kTileBytes + (FMT == kInt4 ? 1024 : 0);
   static constexpr int kXBytes = kWarps * kPieces * NT * 8 * 128;
-  static constexpr int kXScaleBytes = FMT == kFp8 ? kWarps * NT * 8 * 4 : 0;
+  static constexpr int kXScaleBytes = FMT == kFp8 ? kWarps * 8 * 4 : 0;
   static constexpr int kSlotBytes = (kXBytes + kXScaleBytes + 1023) / 1024 * 1024;
   static constexpr int kSlots = FMT == kInt4 ? (NT == 1 ? 3 : 2) : (NT == 1 ? 4 : NT == 2 ? 3 : 2);
   static constexpr int kRedFloats = kBlocks * kRows * NT * 8;     // of one warp; half of the warps write at a time
   static constexpr int kFixed = kSlots * kSlotBytes + kWarps / 2 * kRedFloats * 4 + 1024 + 512;
   static constexpr int kStages = (kSmemMax - kFixed) / kStageBytes < 12 ? (kSmemMax - kFixed) / kStageBytes : 12;
   static constexpr int kSmem = kFixed + kStages * kStageBytes;
+  static_assert(FMT != kFp8 || NT == 1, "fp8 takes up to eight tokens");
   static_assert(kStages >= 6 && (2 * kStages + 2 * kSlots) * 8 <= 512, "carve-up of the shared memory");
 };
 
@@ -367,7 +368,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
                 }
               }
               if (FMT == kFp8) {
-                sx[j] = lds_f2(xs + C::kXBytes + (warp * NT * 8 + j * 8 + 2 * q) * 4);
+                sx[j] = lds_f2(xs + C::kXBytes + (warp * 8 + 2 * q) * 4);
                 seen |= __float_as_uint(sx[j].x);
               }
             }
@@ -587,7 +588,7 @@ int launch_nt(const Operands& o, const Args& a, int max_ctas, cudaStream_t strea
   if (FMT == kFp8) {
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(a.M), static_cast<cuuint64_t>(a.K / 128)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(o.xs_pitch) * 4};
-    const cuuint32_t box[2] = {NT * 8, kWarps};
+    const cuuint32_t box[2] = {8, kWarps};
     rc = make_map(&tmS, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, o.xs, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) return rc;
   }
@@ -665,9 +666,12 @@ int skinny_bf16(const void* X, int ldx, const void* W, void* C, const void* bias
 }
 
 // Up to 8 tokens (us, here / tcgen05: 57344 x 8192 79 / 114, 8192 x 28672 44 / 58, 10240 x 8192 22 / 32).  From 9 to 16 tokens it
-// would still be the faster one (91 / 104, 48 / 51, 24 / 31), but activations are quantised anew for every product, so the last bit of a
-// sum can become a sixteenth of a value; the tcgen05 kernels give a prompt of that length the same sums alone and among others, and a
-// prompt's greedy answer is relied on not to depend on what it is batched with.
+// would still be the faster one (91 / 104, 48 / 51, 24 / 31).  The line lies at 8 because activations are quantised anew for every
+// product, so that the last bit of a sum can become a sixteenth of a value: the tcgen05 kernel gives tokens from 9 to 128 the same
+// sums in every batch, and with the line at 16 a short prompt that was sent alone and then four times at once got other greedy
+// answers.  A prompt of up to 8 tokens (or such a rest of one) and a decode step of up to 8 sequences don't have that: among more
+// tokens their sums have another order.  In bf16 and with 4-bit weights the order changes with the number of tokens, too, but a last
+// bit stays one.
 bool skinny_fp8_applies(const void* X, const float* xs_t, const void* W, int M, int K) {
   return M <= 8 && K % 128 == 0 && aligned16(X) && aligned16(xs_t) && aligned16(W);
 }

@@ -304,10 +304,9 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
   const uint32_t sf_ready0_remote = (PAIR && MX) ? map_to_cta(smem_u32(&sf_ready[0]), 0) : 0u;
   // Barrier set-up, TMEM allocation and descriptor prefetch above touch no tensor data, so they overlap
   // with the tail of the previous kernel; from here on the operands (and the workspace) are used.  Settled weights
-  // (gemm_skinny.h) fill the ring before that: the producer waits behind them.  Decode steps: 8B 201 sequences 5404 -> 5323 us,
-  // 70B fp8 256 sequences 4350 -> 4269, Mixtral 48 sequences 2435 -> 2389.
+  // (gemm_skinny.h) fill the ring before that: the producer waits behind them.  Decode steps without it / with it, us: 8B 201 sequences
+  // 5475 / 5423, 70B fp8 256 sequences 4395 / 4353, Mixtral 48 sequences 2464 / 2433.
   if (warp != 0 || !settled) tgi::pdl_wait();
-  tgi::pdl_trigger();
 
   if (warp < 4) {
     reg_dec<40>();
@@ -841,9 +840,9 @@ int launch(const void* X, const float* xs_t, int xs_pitch, const void* W, const 
   if (grid < 1) grid = 1;
   int whole_tiles = 0;
   if (tiles > max_workers && !(FP8 && M > Cfg::TM)) {
-    // Whole tiles in rounds, or equal shares whose cut tiles are put together through global memory, which costs 10 to 20 us.  How many
-    // K blocks of 128 bytes that is depends on what a worker needs for one: 0.2 us in bf16, 0.4 in block-scaled fp8 on pairs, 0.6 in fp8
-    // with promotion.  Measured on B200, captured, equal shares / whole tiles in us at the blocks that the latter take on top:
+    // Whole tiles in rounds, or equal shares whose cut tiles are put together through global memory, which costs 10 to 20 us.  A K block
+    // (128 bytes) that whole tiles take on top costs 0.2 us in bf16, 0.4 in block-scaled fp8 on pairs, 0.6 in fp8 with promotion, less on
+    // single CTAs of few tokens.  Measured on B200, captured, equal shares / whole tiles in us at the blocks that the latter take on top:
     //   bf16 pairs, 201 tokens         28672 x 4096  (31) 66 / 56     19200 x 4096 (63) 52 / 49      57344 x 8192 (124) 242 / 264
     //   bf16, 64 tokens                128256 x 4096 (39) 182 / 170   57344 x 8192 (62) 163 / 153    38400 x 8192 (126) 114 / 115
     //   fp8 block-scaled, 201 tokens   28672 x 4096  (15) 54 / 41     28672 x 8192 (31) 78 / 70      57344 x 8192 (62) 150 / 162
@@ -862,7 +861,7 @@ int launch(const void* X, const float* xs_t, int xs_pitch, const void* W, const 
   }
   if (tiles <= max_workers) {
     // Rough costs in microseconds, from timelines measured on B200: a K block takes about 0.4 us per
-    // CTA; every partial tile costs 128 KB written and read through L2 by all CTAs at once (about
+    // CTA (all of them are at work, which those of a last, partly filled round are not); every partial tile costs 128 KB written and read through L2 by all CTAs at once (about
     // 0.05 us each at ~5 TB/s) and a split adds ~3 us of publish / wait / reduce latency.
     const double kUnit = 0.4, kPartial = 0.05, kSync = 3.0;
     const double partials_sk = static_cast<double>(grid + tiles < 2 * grid ? grid + tiles : 2 * grid);

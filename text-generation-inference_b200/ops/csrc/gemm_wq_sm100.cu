@@ -113,7 +113,6 @@ gemm_wq_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
   tgi::pdl_wait();
-  tgi::pdl_trigger();
 
   // unit -> (tile coordinates, K-block range); the weight tile is the slow index so that the CTAs working at
   // the same time stream different weight rows and share the token tiles in L2
@@ -392,7 +391,6 @@ gemm_wq_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ 
 __global__ void __launch_bounds__(256)
 wq_cast_kernel(const __nv_bfloat16* __restrict__ x, __half* __restrict__ y, long long vecs) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   for (long long v = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; v < vecs;
        v += static_cast<long long>(gridDim.x) * blockDim.x) {
     const uint4 raw = reinterpret_cast<const uint4*>(x)[v];

@@ -330,7 +330,6 @@ latent_attention_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     tmem_relinquish();
   }
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   if (p.persistent) {
     decode_tiles(p, prefix);
     __syncthreads();
@@ -658,7 +657,6 @@ template <int N>
 __global__ void __launch_bounds__(128)
 latent_merge_kernel(const LatentParams p) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   constexpr int kBatch = 128;                              // parts whose weights are held at a time
   __shared__ float s_f[kBatch];
   __shared__ float red[8];

@@ -1,16 +1,16 @@
 // Kernel launch helper with optional programmatic dependent launch (PDL).
 //
 // A decode step is several hundred short kernels replayed from a CUDA graph.  With PDL a kernel is
-// launched with the "programmatic stream serialization" attribute and starts with `pdl_wait()` (which
-// blocks until the kernels it depends on have completed and flushed their memory) followed by
-// `pdl_trigger()`, so the next kernel's CTAs can be placed on the SMs while this one is still
-// running.  Nothing is read or written before `pdl_wait()`, so stream-order semantics are preserved (but for settled weights,
-// see `pdl_release`).
+// launched with the "programmatic stream serialization" attribute and starts with `pdl_wait()`, which
+// blocks until the kernels it depends on have completed and flushed their memory; its launch and what it does before
+// that overlap with their ends.  Nothing is read or written before `pdl_wait()`, so stream-order semantics are preserved (but for
+// settled weights, see `pdl_release`).
 //
-// Measured on B200 (CUDA-graph decode step): Llama-3-70B fp8 at TP=1 56.6 ms with PDL against 56.4 ms
-// without, TP=2 35.4 against 34.8 ms, Llama-3-8B bf16 at TP=2 10.7 against 10.4 ms.  Inside a graph the
-// launch gaps are already small and the early-placed CTAs only take resources, so the attribute is
-// OFF by default; `TGI_B200_PDL=1` switches it on (the device-side calls are no-ops without it).
+// The attribute is always set on GEMMs that fetch settled weights; `TGI_B200_PDL=1` sets it on all launches, which gains next to
+// nothing inside a graph, where launch gaps are already small.  Steps on B200 without / with it, us: 8B bf16 19 sequences
+// 2185 / 2179, 201 sequences 5458 / 5453, 70B fp8 256 sequences 4403 / 4404 (8 layers), 8B 4-bit 12 sequences 1784 / 1769;
+// over two GPUs, where kernels wait for the other rank's, it cost 2 to 3 % (70B fp8 34.8 / 35.4 ms, 8B 10.4 / 10.7).  Hence off by default.
+// Without the attribute the device-side calls do nothing.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -20,19 +20,13 @@
 namespace tgi {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Early trigger: lets the dependent grid be placed while this one still runs.  Measured slower (the early CTAs
-// take SM slots from later waves of the running kernel), so by default the trigger is the implicit one at CTA
-// exit and only the launch latency and the prologue of the next kernel overlap with this kernel's tail.
-__device__ __forceinline__ void pdl_trigger() {
-#ifdef TGI_PDL_EARLY_TRIGGER
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#endif
-}
 
-// The trigger of the short kernels that a decode step's GEMMs follow (norm, activation, quantisation, decode attention): such a
-// GEMM may be launched so that it fetches settled weights meanwhile (`launch_after`), and its CTAs take nothing that these
-// kernels' later CTAs need, since all of those have started when the trigger takes effect.  Comes after `pdl_wait()`, so that what
-// runs ahead of its own wait runs after everything but its direct predecessor.
+// Kernels trigger their dependents implicitly, when they end: with a trigger at entry everywhere the early CTAs take SM slots from
+// later waves of the running kernel (a step of 19 sequences on an 8B model 2255 -> 2427 us).  This is the explicit trigger of the
+// short kernels that a decode step's GEMMs follow (norm, activation, quantisation, decode attention): such a GEMM may be launched so
+// that it fetches settled weights meanwhile (`launch_after`), and its CTAs take nothing that these kernels' later CTAs need, since all
+// of those have started when the trigger takes effect.  Comes after `pdl_wait()`, so that what runs ahead of its own wait runs after
+// everything but its direct predecessor.
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 inline bool pdl_enabled() {

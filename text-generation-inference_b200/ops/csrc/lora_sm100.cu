@@ -31,7 +31,6 @@ lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, const long long* __restr
                    const int* __restrict__ ranks, const int* __restrict__ token_adapter, float* __restrict__ v, int H,
                    int rmax) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int t = blockIdx.x;
   const int a = token_adapter[t];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -67,7 +66,6 @@ lora_expand_kernel(const float* __restrict__ v, const long long* __restrict__ b_
                    const float* __restrict__ scales, const int* __restrict__ token_adapter,
                    __nv_bfloat16* __restrict__ out, long long out_stride, int col0, int N, int rmax) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   __shared__ float sv[kMaxRank];
   const int t = blockIdx.x;
   const int a = token_adapter[t];

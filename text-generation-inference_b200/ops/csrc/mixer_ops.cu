@@ -44,7 +44,6 @@ template <typename T, int VPT>
 __global__ void __launch_bounds__(1024)
 residual_norm_kernel(ResidualNorm<T> p) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   __shared__ float red[33];
   const int row = p.rows != nullptr ? p.rows[blockIdx.x] : blockIdx.x, H = p.H;
   const size_t in = static_cast<size_t>(row) * H, ob = static_cast<size_t>(blockIdx.x) * H;
@@ -132,7 +131,6 @@ __global__ void __launch_bounds__(256)
 embed_residual_kernel(const int* __restrict__ ids, const T* __restrict__ table, float* __restrict__ out, int H, int vocab,
                       float scale) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int id = min(max(ids[blockIdx.x], 0), vocab - 1);
   const T* src = table + static_cast<size_t>(id) * H;
   float* dst = out + static_cast<size_t>(blockIdx.x) * H;
@@ -164,7 +162,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 act_mul_any_kernel(const T* __restrict__ in, T* __restrict__ out, long long n, int I, int act) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
     const long long t = i / I, c = i - t * I;
@@ -176,7 +173,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 activation_kernel(const T* __restrict__ in, T* __restrict__ out, long long n, int act) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   const long long first = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const long long n4 = n / 4;
@@ -283,7 +279,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 conv_state_kernel(const T* __restrict__ proj, long long ld, int n0, int n1, int off0, int off1, int off2, ConvPast p) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int b = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = p.cu[b + 1] - p.cu[b], slot = p.slots[b];
   if (c >= p.C || n <= 0 || slot < 0 || slot >= p.num_slots) return;
@@ -317,7 +312,6 @@ attn_prep_kernel(const T* __restrict__ proj, long long ld, int off_k, int off_v,
                  int T_, int Hq, int Hkv, int dim, int vdim, int Dk, int Dv, int rot, int max_pos,
                  long long num_slots, int qk_norm, float eps, int inter, ConvPast cv) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int heads = Hq + 2 * Hkv;
   const long long job = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -401,7 +395,6 @@ attn_prep_vec_kernel(const T* __restrict__ proj, long long ld, int off_k, int of
                      T* __restrict__ v_cache, int Hq, int Hkv, int dim, int vdim, int Dk, int Dv, int rot, int max_pos,
                      long long num_slots, int qk_norm, float eps) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int t = blockIdx.x, l = threadIdx.x & 15;
   const long long slot = slots[t];
   const bool slot_ok = slot >= 0 && slot < num_slots;
@@ -477,7 +470,6 @@ attn_conv_run_kernel(const T* __restrict__ proj, long long ld, int off_k, int of
                      T* __restrict__ k_cache, T* __restrict__ v_cache, int T_, int Hq, int Hkv, int dim, int vdim, int Dk, int Dv,
                      int rot, int max_pos, long long num_slots, int qk_norm, float eps, int run, ConvPast cv) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int l = threadIdx.x % L;
   const int h = blockIdx.y * (blockDim.x / L) + threadIdx.x / L;
   const bool on = h < Hq + 2 * Hkv;                        // lanes past the last head stay for the exchanges
@@ -619,7 +611,6 @@ attn_any_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T*
                 T* __restrict__ out, int T_, int B, int max_blocks, int bs_shift, int Hq, int Hkv, int Dk, int Dv, int ldv,
                 AnyAttention<T> a) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   extern __shared__ float sq[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float* qs = sq + warp * Dk;
@@ -723,7 +714,6 @@ delta_prep_kernel(const T* __restrict__ proj, const T* __restrict__ a_pre, const
                   float* __restrict__ k_out, float* __restrict__ v_out, float* __restrict__ g_out,
                   float* __restrict__ beta_out, float* __restrict__ qk_out, int T_, int num_slots, DeltaPrep p) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int units = p.G + (p.head_decay ? 1 : 2) * p.H;
   const long long job = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -821,7 +811,6 @@ delta_prep_run_kernel(const T* __restrict__ proj, const T* __restrict__ a_pre, c
                       float* __restrict__ g_out, float* __restrict__ beta_out, float* __restrict__ qk_out, int T_,
                       int num_slots, int run, DeltaPrep p) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int first = UNITS == 2 ? p.G : (UNITS == 3 ? p.G + p.H : 0);
   const int u = first + blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1034,7 +1023,6 @@ template <typename T, bool ATTN>
 __global__ void __launch_bounds__(256, 2)
 conv_tile_kernel(const T* __restrict__ proj, ConvTile p, ConvPast cv) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   constexpr int TAPS = 4, HALO = TAPS - 1, PER = 16 / sizeof(T);      // elements of a 16-byte piece
   using Out = typename std::conditional<ATTN, T, float>::type;
   __shared__ __align__(16) T tile[kTileRows + HALO][kTileCols];
@@ -1189,7 +1177,6 @@ gated_norm_kernel(const float* __restrict__ o, const T* __restrict__ gate, long 
                   const float* __restrict__ weight, T* __restrict__ out, long long ld_out, int T_, int groups, int width,
                   float eps) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   __shared__ float red[33];
   const int t = blockIdx.x;
   const int g = WARP ? blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5) : blockIdx.y;

@@ -133,7 +133,6 @@ __global__ void __launch_bounds__(32 * WM * WK)
 moe_router_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, int tokens, int E, int K,
                   int k_split, float* __restrict__ part) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   __shared__ float red[WK > 1 ? (WK - 1) * WM : 1][WK > 1 ? NT * 4 : 1][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
   const int wm = warp % WM, wk = warp / WM;
@@ -190,7 +189,6 @@ __global__ void __launch_bounds__(128)
 moe_topk_scores_kernel(const float* __restrict__ part, int parts, const float* __restrict__ correction, int tokens, int E,
                         int k, float scale, float* __restrict__ out_w, int* __restrict__ out_ids) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (t >= tokens) return;
@@ -347,7 +345,6 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ 
 __global__ void __launch_bounds__(256)
 moe_combine_f32_kernel(const float* __restrict__ y, const int* __restrict__ pos, int tokens, int k, int H, float* __restrict__ out) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   for (int t = blockIdx.x; t < tokens; t += gridDim.x)
     for (int i = threadIdx.x; i < H; i += blockDim.x) {
       float acc = 0.f;
@@ -445,7 +442,6 @@ moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     tmem_relinquish();
   }
   tgi::pdl_wait();      // the counts come from the sort kernel before this one
-  tgi::pdl_trigger();
   if (threadIdx.x == 32) {
     int run = 0;
     for (int e = 0; e < e_local; ++e) {
@@ -641,7 +637,6 @@ moe_grouped_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
                        const int* __restrict__ order, int e_local, int k, int Nw, int K, int act,
                        const float* __restrict__ topk_w, float* __restrict__ out) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   constexpr int P = MODE == 0 ? 2 : 1;                     // products per output
   __shared__ float sa[16][68], sw[P][16][68];
   int tile = blockIdx.y, e = 0;

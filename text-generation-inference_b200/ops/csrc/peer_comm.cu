@@ -233,7 +233,6 @@ peer_reduce_kernel(const PeerArgs a) {
   __shared__ float red[32];
   __shared__ int failed;
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   if (threadIdx.x == 0) failed = 0;
   __syncthreads();
   BlockSync sync(a, &failed);
@@ -371,7 +370,6 @@ peer_argmax_kernel(const PeerArgs a, const __nv_bfloat16* __restrict__ logits, l
   __shared__ int sm_i[32];
   __shared__ int failed;
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   if (threadIdx.x == 0) failed = 0;
   __syncthreads();
   BlockSync sync(a, &failed);
@@ -470,7 +468,7 @@ peer_argmax_kernel(const PeerArgs a, const __nv_bfloat16* __restrict__ logits, l
 // Vocabulary-parallel sampling.  The reference gathers the [B, V] logits of the sharded lm_head on every rank
 // and runs its warper chain on the full matrix (layers/tensor_parallel.py:75-104, utils/tokens.py:233-503).
 // Here every rank keeps its [B, V / world] slice and the ranks agree on the result through a few scalars per
-// row: the fused single-GPU sampler (fused_ops.cu `sample_kernel`) only ever needs block-wide reductions of the
+// row: the fused single-GPU sampler (sampler.cu `sample_kernel`) only ever needs block-wide reductions of the
 // row (max, counts and probability mass above a threshold, the arg-max of the Gumbel-perturbed scores), so each
 // of them becomes a block reduction over the slice followed by an exchange of one 8-byte word per rank.
 //
@@ -589,7 +587,6 @@ peer_sample_kernel(const PeerArgs a, const SampleArgs sa, const T* __restrict__ 
   __shared__ int s_idx[32];
   __shared__ int failed;
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   if (threadIdx.x == 0) failed = 0;
   __syncthreads();
   Exchange xc{a, sa.off_xchg, sa.xseq[blockIdx.x], &failed, recv};

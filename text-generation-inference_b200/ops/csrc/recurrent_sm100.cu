@@ -193,7 +193,6 @@ __global__ void __launch_bounds__(kThreads)
 scan_kernel(ScanArgs p) {
   constexpr bool DELTA = is_delta(MODE), WIDE = MODE == kChannel, HEAD = MODE == kHead;
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   extern __shared__ __align__(16) float smem[];
   using S = ScanCfg<MODE, J, L, CN>;
   constexpr int kItems = 64 * J;                                // (block, channel pair) items of a tile
@@ -537,7 +536,6 @@ __global__ void __launch_bounds__(kThreads)
 step_kernel(ScanArgs p) {
   constexpr bool DELTA = is_delta(MODE), HEAD = MODE == kHead;
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int b = blockIdx.z, h = blockIdx.y;
   const int t = p.cu[b];
   if (p.cu[b + 1] <= t) return;

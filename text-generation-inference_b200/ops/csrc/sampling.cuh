@@ -1,4 +1,4 @@
-// Device helpers shared by the single-GPU sampler (fused_ops.cu) and the vocabulary-parallel sampler
+// Device helpers shared by the single-GPU sampler (sampler.cu) and the vocabulary-parallel sampler
 // (peer_comm.cu): order-preserving integer image of a float, Philox4x32-10 and the Gumbel noise of entry j.
 #pragma once
 #include <cuda_runtime.h>

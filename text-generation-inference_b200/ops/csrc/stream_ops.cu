@@ -96,7 +96,6 @@ template <typename T, int VPT, int CONV, bool AVG>
 __global__ void __launch_bounds__(CONV > 0 ? 1024 : 512, CONV > 0 ? 1 : 2)
 stream_step_kernel(const StreamStep<T> p) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   __shared__ float red[2][33];
   extern __shared__ float held[];                          // VPT == 0: [H]
   const int row = p.rows != nullptr ? p.rows[blockIdx.x] : blockIdx.x, H = p.H;
@@ -299,7 +298,6 @@ template <typename T, int TAPS, int R>
 __global__ void __launch_bounds__(128)
 input_conv_kernel(const T* __restrict__ x, T* __restrict__ out, int T_, int H, const InputConv p) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   constexpr int Q = Piece<T>::Q;
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * Q, t0 = blockIdx.y * R, t1 = min(T_, t0 + R);
   if (c >= H) return;
@@ -364,7 +362,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 input_conv_any_kernel(const T* __restrict__ x, T* __restrict__ out, int H, const InputConv p) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int c = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y;
   if (c >= H) return;
   const int b = sequence_of(p.cu, p.B, t), begin = p.cu[b], local = t - begin, slot = p.slots[b];
@@ -386,7 +383,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 input_conv_state_kernel(const T* __restrict__ x, int H, const InputConv p) {
   tgi::pdl_wait();
-  tgi::pdl_trigger();
   const int b = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
   const int begin = p.cu[b], n = p.cu[b + 1] - begin, slot = p.slots[b];
   if (c >= H || n <= 0 || slot < 0 || slot >= p.num_slots) return;
