@@ -58,7 +58,9 @@ struct Cfg {
   static constexpr int kUnitK = FMT == kBf16 ? 64 : 128;          // features of a unit
   static constexpr int kUnits = FMT == kInt4 ? 2 : 1;             // units in 128 bytes of a weight row
   static constexpr int kPieces = FMT == kInt4 ? 2 : 1;            // 128-byte pieces of a token in a unit
-  static constexpr int kChains = NT == 1 ? 2 : 1;                 // MMA chains of a unit with scales of its own
+  // MMA chains of a unit with scales of its own.  4-bit: one whatever the tokens, so that a token's sums are the same in every
+  // instance (two for up to 8 tokens: 28672 x 4096 29.3 us, one 28.9)
+  static constexpr int kChains = FMT == kFp8 ? 2 : 1;
   static constexpr int kXRegs = FMT == kBf16 ? 8 : 16;            // B fragments of a unit, per 8 tokens
   static constexpr int kScaleBytes = FMT == kInt4 ? 16 * kRows * 2 : 0;               // of a stage, zero points as many
   static constexpr int kStageBytes = kTileBytes + (FMT == kInt4 ? 1024 : 0);
@@ -670,8 +672,8 @@ int skinny_bf16(const void* X, int ldx, const void* W, void* C, const void* bias
 // product, so that the last bit of a sum can become a sixteenth of a value: the tcgen05 kernel gives tokens from 9 to 128 the same
 // sums in every batch, and with the line at 16 a short prompt that was sent alone and then four times at once got other greedy
 // answers.  A prompt of up to 8 tokens (or such a rest of one) and a decode step of up to 8 sequences don't have that: among more
-// tokens their sums have another order.  In bf16 and with 4-bit weights the order changes with the number of tokens, too, but a last
-// bit stays one.
+// tokens their sums have another order.  In bf16 and with 4-bit weights a token's sums are the same in all batches that come here and
+// others in larger ones, but there a last bit stays one.
 bool skinny_fp8_applies(const void* X, const float* xs_t, const void* W, int M, int K) {
   return M <= 8 && K % 128 == 0 && aligned16(X) && aligned16(xs_t) && aligned16(W);
 }
@@ -696,9 +698,8 @@ int skinny_int4(const void* X, const void* W, const void* scale, const void* zp,
                        M - m0 < kInt4Tokens ? M - m0 : kInt4Tokens, N, K, settled && m0 == 0, status);
     a.has_zp = zp != nullptr;
     a.group_units = group / 128;
-    const Operands o{static_cast<const __nv_bfloat16*>(X) + static_cast<size_t>(m0) * K, 2LL * K, W, nullptr, 0, scale, zp};
-    // all tokens of a call in the same chains of MMAs: equal tokens give equal rows
-    const int rc = M > kInt4Tokens ? launch_nt<kInt4, 2>(o, a, max_ctas, stream) : launch<kInt4>(o, a, max_ctas, stream);
+    const int rc = launch<kInt4>(Operands{static_cast<const __nv_bfloat16*>(X) + static_cast<size_t>(m0) * K, 2LL * K, W, nullptr, 0,
+                                          scale, zp}, a, max_ctas, stream);
     if (rc) return rc;
   }
   return 0;
