@@ -1,8 +1,8 @@
 """Shares of the persistent GEMM (``ops/csrc/gemm_sm100.cu``): whole tiles in rounds, equal shares with cut tiles, and K splits, with
 even and uneven rounds, ragged edges and few CTAs, in both tile shapes and on CTA pairs, in bf16 and in both modes of fp8.
 
-Tolerance: one rounding to bf16 (2^-8 of the value at most) and fp32 sums (2^-24 per addition, at most 2^14 of them, of the
-products' magnitudes)."""
+Tolerance: one rounding to bf16 (2^-8 of the value at most) and fp32 sums, which the tensor core rounds once per 16 features (2^-23
+of the products' magnitudes each, at most 2^10 times); a K block that is missing or met twice is several times that."""
 import pytest
 import torch
 
@@ -32,7 +32,7 @@ def test_shares(M, N, Kd, ctas, pairs):
     assert K.check_status(dev) == 0, "a kernel wait timed out"
     xd, wd = x.double(), w.double()
     want = xd @ wd.t() + bias.double()
-    assert ((got.double() - want).abs() <= want.abs() * 2 ** -8 + (xd.abs() @ wd.abs().t() + 1) * 2 ** -10).all()
+    assert ((got.double() - want).abs() <= want.abs() * 2 ** -8 + (xd.abs() @ wd.abs().t() + 1) * 2 ** -13).all()
 
 
 @pytest.fixture
